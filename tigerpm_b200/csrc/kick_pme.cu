@@ -18,13 +18,12 @@
 //    memory as float offsets from the sink cell centre: the int32
 //    wrap-around difference (the reference's periodic minimum image) is taken
 //    once per source per block, so the pair loop is pure FP32.
-//  * Culling: the cell's sinks (up to 256 per pass) are ordered by a 9-bit
-//    Morton key of their position inside the cell (a deterministic bitonic
-//    sort) and cut into groups of 8; a warp keeps the sources within the
-//    cutoff of a group's bounding box (ballot + popc) in a float4 buffer, and
-//    lanes (8 sinks x 4 source phases) evaluate it 32 sources at a time,
-//    every lane together: the flush is a warp-uniform branch, pairs go two at
-//    a time with one warp vote for the softened kernel.
+//  * Culling: the cell's sinks (up to 256 per pass) are cut into compact
+//    groups of 8 by halving along x, y, z in turn; a warp keeps the sources
+//    within the cutoff of a group's bounding box (ballot + popc) in a ring
+//    buffer, and lanes (8 sinks x 4 source phases) evaluate it 64 sources at a
+//    time, every lane together: the flush is a warp-uniform branch, pairs go
+//    four at a time in packed FP32 with one warp vote for the softened kernel.
 //  * Pair terms: rsqrt / rcp / ex2 approximations (MUFU) for 1/r, the A&S
 //    rational and exp(-x^2), with lengths in units of 2 r_s / sqrt(log2 e)
 //    so that exp(-x0^2) = 2^-r2; an optional cutoff zeroes pairs beyond it.
@@ -78,12 +77,14 @@ struct KickArgs {
   int first_call;
   int kahan;
   float GM, eta, t0, scale, hsoft;
-  // pair-loop lengths are in units of u = 2 r_s / sqrt(log2 e) (see pair())
+  // pair-loop lengths are in units of u = 2 r_s / sqrt(log2 e) (see pairs())
   float inv2rs;  // 1 / (2 r_s), box units
   float lscale;  // 2^-32 / u: fixed32 offset -> scaled length
   float h2;      // (hsoft / u)^2
   float rcut2;   // (r_cut / u)^2, or infinity without a cutoff
   float wlen;    // the box length / u (minimum-image fold, chain_dim = 3)
+  float cull_k;  // u / r_cut: scaled length -> cutoffs (0 without a cutoff)
+  float cull_m;  // rounding margin of the cull, in cutoffs
 };
 
 __device__ __forceinline__ void kahan_add(float& s, float& c, float v) {
@@ -361,51 +362,17 @@ __global__ void __launch_bounds__(128) k_interp_tile(KickArgs a, int maxw) {
 // Pair constants that stay in registers through the pair loop, in the pair
 // loop's length unit u (below): rcut2 and h2 are (r_cut / u)^2 and (h / u)^2;
 // wrap_len is the box length in u (minimum-image fold, chain_dim = 3 only).
+// A&S 7.1.26: erfc(x) = (a1 t + .. + a5 t^5) exp(-x^2), t = 1 / (1 + p x); in the
+// pair loop t' = 1 / (1/p' + r) with p' = p / sqrt(log2 e), so t = t' / p' and
+// the coefficients are a_k / p'^k.
+constexpr double kP = 0.3275911 / 1.2011224087864498;
+constexpr float kInvP = (float)(1.0 / kP), kA1 = (float)(0.254829592 / kP), kA2 = (float)(-0.284496736 / (kP * kP)),
+                kA3 = (float)(1.421413741 / (kP * kP * kP)), kA4 = (float)(-1.453152027 / (kP * kP * kP * kP)),
+                kA5 = (float)(1.061405429 / (kP * kP * kP * kP * kP));
 constexpr float kLog2e = 1.4426950408889634f, kSqrtLog2e = 1.2011224087864498f;
 struct PairK {
   float rcut2, h2, wrap_len;
 };
-
-// One source against one sink (src/kick_pme.cu:285-314), in three parts:
-// the separation and the erfc-split terms, the softened kernel, and the
-// sums.  WRAP folds the offset to the minimum image, as the reference's
-// int32 difference does; it is needed only when chain_dim = 3, where the 27
-// cells span the whole box and an offset from the cell centre can exceed
-// half the box.
-//
-// Lengths are in units of u = 2 r_s / s with s = sqrt(log2 e) (the caller
-// scales offsets by 1 / u): r2 = log2(e) x0^2 for x0 = r / (2 r_s), so
-// exp(-x0^2) = 2^-r2 takes no multiply.  With x0 = r / s the A&S and
-// 2/sqrt(pi) constants are divided by s, and the sums come out as force x
-// u^2 and potential x u; the caller multiplies them back.  The softened
-// terms are homogeneous in r and h, so their formulas are unchanged.
-template <bool WRAP>
-__device__ __forceinline__ void pair_terms(const PairK& k, float& dx, float& dy, float& dz, float& r2, float& rinv3,
-                                           float& q) {
-  if (WRAP) {
-    const float inv = 1.0f / k.wrap_len;
-    dx -= rintf(dx * inv) * k.wrap_len;
-    dy -= rintf(dy * inv) * k.wrap_len;
-    dz -= rintf(dz * inv) * k.wrap_len;
-  }
-  r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  // Pairs beyond the cutoff take r^2 = 1e30: 1/r, erfc and exp(-x^2) then
-  // vanish and the pair adds exactly 0, without a mask on the results.
-  // Pairs at r <= h (the sink itself included, r = 0) take the softened
-  // kernel, which replaces every term formed here.
-  const float r2c = r2 < k.rcut2 ? r2 : 1e30f;
-  const float rinv = rsqrt_approx(r2c);
-  const float r = r2c * rinv;
-  // A&S 7.1.26 erfc(x0), t = 1 / (1 + 0.3275911 x0) with x0 = r / s
-  const float t = rcp_approx(fmaf(0.2727374808792225f, r, 1.0f));
-  const float e = ex2_approx(-r2c);
-  const float poly =
-      t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
-  // potential term erfc / r, and the force term
-  // (erfc + (2/sqrt(pi)) x0 e) / r^3 = (erfc / r + (2/sqrt(pi)) e / s) / r^2
-  q = poly * e * rinv;
-  rinv3 = fmaf(0.9394372786996513f, e, q) * (rinv * rinv);
-}
 
 // The softened Newtonian kernel where r <= h (rare), selected per lane.
 __device__ __forceinline__ void soften(const PairK& k, float r2, float& rinv3, float& q) {
@@ -418,41 +385,94 @@ __device__ __forceinline__ void soften(const PairK& k, float r2, float& rinv3, f
   q = soft ? s1 : q;
 }
 
-__device__ __forceinline__ void add_pair(float dx, float dy, float dz, float rinv3, float q, float& gx, float& gy,
-                                         float& gz, float& ph) {
-  gx = fmaf(-dx, rinv3, gx);
-  gy = fmaf(-dy, rinv3, gy);
-  gz = fmaf(-dz, rinv3, gz);
-  ph -= q;
-}
-
-// One pair, the softened kernel behind a per-lane branch (any caller).
-template <bool WRAP>
-__device__ __forceinline__ void pair(const PairK& k, float dx, float dy, float dz, float& gx, float& gy, float& gz,
-                                     float& ph) {
-  float r2, rinv3, q;
-  pair_terms<WRAP>(k, dx, dy, dz, r2, rinv3, q);
-  if (r2 <= k.h2) soften(k, r2, rinv3, q);
-  add_pair(dx, dy, dz, rinv3, q, gx, gy, gz, ph);
-}
-
-// Two pairs of one sink, evaluated by every lane of the warp together: the
-// softened kernel is entered on one warp vote for both (a uniform branch),
-// and the sums take the first pair, then the second.
-template <bool WRAP>
-__device__ __forceinline__ void pair2(const PairK& k, const float4& sp, const float4 u0, const float4 u1, float& gx,
-                                      float& gy, float& gz, float& ph) {
-  float dx0 = sp.x - u0.x, dy0 = sp.y - u0.y, dz0 = sp.z - u0.z;
-  float dx1 = sp.x - u1.x, dy1 = sp.y - u1.y, dz1 = sp.z - u1.z;
-  float r20, rinv30, q0, r21, rinv31, q1;
-  pair_terms<WRAP>(k, dx0, dy0, dz0, r20, rinv30, q0);
-  pair_terms<WRAP>(k, dx1, dy1, dz1, r21, rinv31, q1);
-  if (__any_sync(0xffffffffu, r20 <= k.h2 || r21 <= k.h2)) {
-    soften(k, r20, rinv30, q0);
-    soften(k, r21, rinv31, q1);
+// 2 NP sources against one sink (src/kick_pme.cu:285-314), two per packed
+// FP32 instruction.  The pair loop is bound by the issue slots, the FP32 pipe
+// (a packed instruction of three different operands takes it 3 cycles, a
+// scalar one 1.5) and the MUFU (8 cycles a result and warp, 3 results a pair)
+// about equally: in isolation 16 sources x 8 sinks take a warp 89 instructions
+// and 137 cycles of an SM quarter, 130 and 157 as scalars.  Kick at 256^3:
+// 14.30 -> 13.43 ms on the 768^3 mesh, 41.6 -> 33.1 ms on the literal mesh;
+// 88.0 -> 67 ms for the reference's options at 90^3 (packed pairs, groups by
+// halves and the 64-source cull step together).
+//
+// WRAP folds the offset to the minimum image, as the reference's int32
+// difference does; it is needed only when chain_dim = 3, where the 27 cells
+// span the whole box and an offset from the cell centre can exceed half the
+// box (rounded by adding and subtracting 1.5 x 2^23, exact to-nearest-even for
+// these |x| < 2).
+//
+// Lengths are in units of u = 2 r_s / s with s = sqrt(log2 e) (the caller
+// scales offsets by 1 / u): r2 = log2(e) x0^2 for x0 = r / (2 r_s), so
+// exp(-x0^2) = 2^-r2 takes no multiply.  With x0 = r / s the A&S and
+// 2/sqrt(pi) constants are divided by s, and the sums come out as force x
+// u^2 and minus the potential x u; the caller multiplies them back.  The
+// softened terms are homogeneous in r and h, so their formulas are unchanged.
+//
+// ns is minus the sink, s the sources, sum the packed partial sums (even and
+// odd sources apart).  Every lane of the warp calls it together: the softened
+// kernel (r <= h, the sink itself included) is entered on one warp vote.
+// count: sources from this lane's first one on that exist (WRAP only; without
+// it the caller pads with far sources).
+template <bool WRAP, int NP>
+__device__ __forceinline__ void pairs(const PairK& k, const f32x2 (&ns)[3], const f32x2 (&s)[3][NP], f32x2 (&sum)[4],
+                                      int count) {
+  f32x2 d[3][NP], f[NP], q[NP];
+  float r2[2 * NP];
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      d[a][i] = add2(s[a][i], ns[a]);
+      if (WRAP) {
+        const float iw = 1.0f / k.wrap_len;
+        const f32x2 m = pack2(12582912.0f, 12582912.0f), nm = pack2(-12582912.0f, -12582912.0f);
+        const f32x2 turns = add2(fma2(d[a][i], pack2(iw, iw), m), nm);
+        d[a][i] = fma2(turns, pack2(-k.wrap_len, -k.wrap_len), d[a][i]);
+      }
+    }
+    const float2 t = unpack2(fma2(d[0][i], d[0][i], fma2(d[1][i], d[1][i], mul2(d[2][i], d[2][i]))));
+    r2[2 * i] = WRAP && count <= 2 * i ? 1e30f : t.x;
+    r2[2 * i + 1] = WRAP && count <= 2 * i + 1 ? 1e30f : t.y;
   }
-  add_pair(dx0, dy0, dz0, rinv30, q0, gx, gy, gz, ph);
-  add_pair(dx1, dy1, dz1, rinv31, q1, gx, gy, gz, ph);
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+    // Pairs beyond the cutoff take r^2 = 1e30: 1/r, erfc and exp(-x^2) then
+    // vanish and the pair adds exactly 0, without a mask on the results.
+    // Pairs at r <= h (r = 0 too) take the softened kernel, which replaces
+    // every term formed here.
+    const float a = r2[2 * i] < k.rcut2 ? r2[2 * i] : 1e30f, b = r2[2 * i + 1] < k.rcut2 ? r2[2 * i + 1] : 1e30f;
+    const f32x2 rinv = pack2(rsqrt_approx(a), rsqrt_approx(b));
+    const float2 w = unpack2(fma2(pack2(a, b), rinv, pack2(kInvP, kInvP)));
+    const f32x2 t = pack2(rcp_approx(w.x), rcp_approx(w.y));
+    const f32x2 e = pack2(ex2_approx(-a), ex2_approx(-b));
+    f32x2 p = fma2(t, pack2(kA5, kA5), pack2(kA4, kA4));
+    p = fma2(t, p, pack2(kA3, kA3));
+    p = fma2(t, p, pack2(kA2, kA2));
+    p = fma2(t, p, pack2(kA1, kA1));
+    // potential term erfc / r, and the force term
+    // (erfc + (2/sqrt(pi)) x0 e) / r^3 = (erfc / r + (2/sqrt(pi)) e / s) / r^2
+    q[i] = mul2(mul2(mul2(t, p), e), rinv);
+    f[i] = mul2(fma2(pack2(0.9394372786996513f, 0.9394372786996513f), e, q[i]), mul2(rinv, rinv));
+  }
+  float least = r2[0];
+#pragma unroll
+  for (int i = 1; i < 2 * NP; i++) least = fminf(least, r2[i]);
+  if (__any_sync(0xffffffffu, least <= k.h2)) {
+#pragma unroll
+    for (int i = 0; i < NP; i++) {
+      float2 fi = unpack2(f[i]), qi = unpack2(q[i]);
+      soften(k, r2[2 * i], fi.x, qi.x);
+      soften(k, r2[2 * i + 1], fi.y, qi.y);
+      f[i] = pack2(fi.x, fi.y);
+      q[i] = pack2(qi.x, qi.y);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NP; i++) {
+#pragma unroll
+    for (int a = 0; a < 3; a++) sum[a] = fma2(d[a][i], f[i], sum[a]);
+    sum[3] = add2(sum[3], q[i]);
+  }
 }
 
 // Offset a - b of two fixed32 coordinates (the reference's int32 wrap-around
@@ -461,39 +481,34 @@ __device__ __forceinline__ float offset_scaled(uint32_t a, uint32_t b, float sc)
   return (float)(int32_t)(a - b) * sc;
 }
 
-// 3-bit-per-axis sub-cell index of an offset (in box units) from the cell
-// centre, interleaved into a 9-bit Morton key.
-__device__ __forceinline__ unsigned morton9(float sx, float sy, float sz, float C) {
-  unsigned q[3];
-  const float s[3] = {sx, sy, sz};
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    const int v = (int)((s[d] * C + 0.5f) * 8.0f);
-    q[d] = (unsigned)min(max(v, 0), 7);
-  }
-  unsigned k = 0;
-#pragma unroll
-  for (int b = 2; b >= 0; b--) k = (k << 3) | (((q[2] >> b) & 1u) << 2) | (((q[1] >> b) & 1u) << 1) | ((q[0] >> b) & 1u);
-  return k;
+// Sort key of a sink along one axis: the upper 24 bits of its place in the
+// cell (offset from the centre o plus half a cell, stretched to 32 bits), and
+// its slot in the pass, which makes keys unique.
+__device__ __forceinline__ unsigned order_key(int x, uint32_t o, int C, int slot) {
+  const long long d = (long long)(int32_t)((uint32_t)x - o) * C + 0x80000000ll;
+  const unsigned u = (unsigned)min(max(d, 0ll), 0xfffffeffll);
+  return (u & 0xffffff00u) | (unsigned)slot;
 }
 
 // Work decomposition.  A block owns one sink cell.  Its active sinks (up to
-// kPass per pass) are sorted by a 9-bit Morton key of their position in the
-// cell, then cut into groups of kGroup = 8 consecutive sinks (compact in
-// space).  Warps take groups round-robin.  For each group a warp streams the
-// staged neighbourhood, keeps the sources within rcut of the group's bounding
-// box (ballot + popc) and copies them contiguously into its float4 buffer;
-// lanes are (sink t = lane % 8) x (phase = lane / 8), so one step evaluates 8
-// sinks against 4 consecutive buffered sources (conflict-free broadcast-free
-// reads) and a fixed two-step shuffle reduction folds the 4 phases.  Per-sink
-// sums live in shared memory with Kahan compensation across chunks.
+// kPass per pass) are cut into groups of kGroup = 8 (compact in space).  Warps take groups round-robin.  For each group a warp streams the
+// staged neighbourhood 64 at a time (two per lane), keeps the sources within
+// rcut of the group's bounding box (ballot + popc) and copies them into its
+// ring buffer; lanes are (sink t = lane % 8) x (phase = lane / 8), so one
+// step evaluates 8 sinks against 16 consecutive buffered sources, 4 per lane,
+// and a fixed two-step shuffle reduction folds the 4 phases.  Sources are
+// staged and buffered as separate x, y and z arrays, so that a 16-byte load
+// gives two packed operands.  Per-sink sums live in shared memory with Kahan
+// compensation across chunks.
 //
-// Shared memory (dynamic): src[stage] float4 | buf[W][kBuf] float4 |
+// Shared memory (dynamic): src[3][stage] float | buf[W][3][kBuf] float |
 // spos[kPass] float4 | acc[kPass][8] float | skey[kPass] | runb/runp.
 constexpr int kPass = 256;
 constexpr int kGroup = 8;
-constexpr int kBuf = 64;
+constexpr int kFlush = 64;        // buffered sources evaluated at a time
+constexpr int kBuf = 2 * kFlush;  // below kFlush left over + 64 appended
 constexpr int kMaxRuns = 18;
+constexpr float kFar = 1e18f;     // offset of a padding source: beyond any cutoff, its terms are exactly 0
 
 // The kick of sink passes [pass_lo, pass_hi) of one sink cell (cx, cy, cz)
 // by the calling block (a pass = the cell's sinks taken np at a time, np =
@@ -504,126 +519,170 @@ template <bool WRAP>
 __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int cz, float4* smem4, int stage,
                                           int npass, int pass_lo = 0, int pass_hi = 0x7fffffff) {
   const int T = blockDim.x, W = T >> 5;
-  float4* src = smem4;
-  float4* bufs = src + stage;
-  float4* spos = bufs + W * kBuf;
+  float* src = reinterpret_cast<float*>(smem4);
+  float* bufs = src + 3 * stage;
+  float4* spos = reinterpret_cast<float4*>(bufs + W * 3 * kBuf);
   float* acc = reinterpret_cast<float*>(spos + npass);
-  unsigned* skey = reinterpret_cast<unsigned*>(acc + npass * 8);
-  int* runb = reinterpret_cast<int*>(skey + npass);
+  unsigned char* sidx = reinterpret_cast<unsigned char*>(acc + npass * 8);
+  int* runb = reinterpret_cast<int*>(sidx + npass);
   int* runp = runb + kMaxRuns;
+  unsigned* mask = reinterpret_cast<unsigned*>(runp + kMaxRuns + 1);
   const int C = a.C;
   const int64_t key = ((int64_t)cz * C + cy) * C + cx;
   const int32_t pb = __ldg(a.begin + key), pe = __ldg(a.begin + key + 1);
   if (pb == pe) return;
-  const uint32_t ox = (uint32_t)((((uint64_t)(2 * cx + 1)) << 31) / (uint64_t)C);
-  const uint32_t oy = (uint32_t)((((uint64_t)(2 * cy + 1)) << 31) / (uint64_t)C);
-  const uint32_t oz = (uint32_t)((((uint64_t)(2 * cz + 1)) << 31) / (uint64_t)C);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int t8 = lane & 7, ph = lane >> 3;
-  const float Cf = (float)C;
   unsigned lt;  // lanes below this one
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
   // offsets, cutoff and softening length in units of 2 r_s / sqrt(log2 e)
-  // (see pair())
-  const float sc = a.lscale;
+  // (see pairs())
   const PairK pk{a.rcut2, a.h2, a.wlen};
   // culling works on unwrapped offsets; without it every source is kept
-  const float keep2 = !WRAP && a.rcut2 < INFINITY ? a.rcut2 : INFINITY;
-  if (tid == 0) {
-    int nr = 0, tot = 0;
-    for (int dz = -1; dz <= 1; dz++) {
-      const int rz = wrapi(cz + dz, C);
-      for (int dy = -1; dy <= 1; dy++) {
-        const int ry = wrapi(cy + dy, C);
-        const int64_t row = ((int64_t)rz * C + ry) * C;
-        int xa[2], xb[2], np;
-        if (cx >= 1 && cx + 1 < C) {
-          xa[0] = cx - 1; xb[0] = cx + 2; np = 1;
-        } else if (cx == 0) {
-          xa[0] = C - 1; xb[0] = C; xa[1] = 0; xb[1] = 2; np = 2;
-        } else {
-          xa[0] = C - 2; xb[0] = C; xa[1] = 0; xb[1] = 1; np = 2;
-        }
-        for (int p = 0; p < np; p++) {
-          const int32_t b = __ldg(a.begin + row + xa[p]), e = __ldg(a.begin + row + xb[p]);
-          runb[nr] = b;
-          runp[nr] = tot;
-          tot += e - b;
-          nr++;
-        }
+  const float ck = WRAP ? 0.f : a.cull_k, cm = WRAP ? 0.f : a.cull_m;
+  uint32_t* org = mask + kPass / 32;  // the cell's centre, not in registers through the pair loop
+  if (tid < 3) org[tid] = (uint32_t)((((uint64_t)(2 * (tid == 0 ? cx : tid == 1 ? cy : cz) + 1)) << 31) / (uint64_t)C);
+  if (warp == 0) {
+    // the neighbourhood's runs: row t / 2 (nine (z, y) rows), part t % 2 (a
+    // row that wraps in x is two runs); lengths to staged offsets by a scan
+    int32_t rb = 0, re = 0;
+    if (lane < kMaxRuns) {
+      const int64_t row = ((int64_t)wrapi(cz + lane / 6 - 1, C) * C + wrapi(cy + lane / 2 % 3 - 1, C)) * C;
+      const bool second = lane & 1;
+      int xa = cx - 1, xb = cx + 2;
+      if (second) {
+        xa = 0;
+        xb = cx == 0 ? 2 : (cx + 1 == C ? 1 : 0);
+      } else if (cx == 0) {
+        xa = C - 1;
+        xb = C;
+      } else if (cx + 1 == C) {
+        xb = C;
       }
+      rb = __ldg(a.begin + row + xa);
+      re = __ldg(a.begin + row + xb);
     }
-    for (int r = nr; r <= kMaxRuns; r++) runp[r] = tot;
+    int incl = re - rb;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane < kMaxRuns) {
+      runb[lane] = rb;
+      runp[lane] = incl - (re - rb);
+    }
+    if (lane == kMaxRuns) runp[kMaxRuns] = incl;  // all lengths past the runs are 0
+  }
+  float* buf = bufs + warp * 3 * kBuf;
+  // Kept in shared memory, not in registers through the pair loop: the sinks
+  // per pass (the power of two >= the cell's count, at most npass) and the end
+  // of this call's passes.
+  if (tid == 0) {
+    int np = 8;
+    while (np < npass && np < pe - pb) np <<= 1;
+    org[3] = np;
+    org[4] = (uint32_t)min((int64_t)pe, (int64_t)pb + (int64_t)pass_hi * np);
+    org[5] = (uint32_t)pe;
   }
   __syncthreads();
-  const int total = runp[kMaxRuns];
-  float4* buf = bufs + warp * kBuf;
-  int np = 8;  // sinks per pass: the power of two >= the cell's count, at most npass
-  while (np < npass && np < pe - pb) np <<= 1;
-  const int32_t s_end = (int32_t)min((int64_t)pe, (int64_t)pb + (int64_t)pass_hi * np);
-  for (int32_t sbase = pb + pass_lo * np; sbase < s_end; sbase += np) {
-    // 1. order this pass's active sinks by sub-cell (deterministic bitonic sort)
-    if (tid == 0) runp[kMaxRuns + 1] = np;  // active count when every slot is active
-    for (int e = tid; e < np; e += T) {
+  for (int32_t sbase = pb + pass_lo * (int)org[3]; sbase < (int32_t)org[4]; sbase += (int)org[3]) {
+    // 1. this pass's active sinks, compacted in slot order ...
+    const int np = (int)org[3], slots = (np + 31) & ~31;
+    for (int e = tid; e < slots; e += T) {
       const int32_t i = sbase + e;
-      unsigned k = 512u;  // inactive / absent sinks sort last
-      if (i < pe && a.rung[i] >= a.min_rung) {
-        const int4 q = __ldg(a.pos4 + i);
-        k = morton9(distance32((uint32_t)q.x, ox), distance32((uint32_t)q.y, oy), distance32((uint32_t)q.z, oz), Cf);
-      }
-      skey[e] = (k << 8) | (unsigned)e;
+      const unsigned m = __ballot_sync(0xffffffffu, e < np && i < (int32_t)org[5] && a.rung[i] >= a.min_rung);
+      if (lane == 0) mask[e >> 5] = m;
     }
-    __syncthreads();
-    for (int kk = 2; kk <= np; kk <<= 1) {
-      for (int j = kk >> 1; j > 0; j >>= 1) {
-        for (int e = tid; e < np; e += T) {
-          const int ixj = e ^ j;
-          if (ixj > e) {
-            const unsigned u = skey[e], v = skey[ixj];
-            const bool up = (e & kk) == 0;
-            if ((u > v) == up) {
-              skey[e] = v;
-              skey[ixj] = u;
+    __syncthreads();  // masks and runs are in place
+    int nact = 0;
+    for (int k = 0; k < slots; k += 32) nact += __popc(mask[k >> 5]);
+    const int ngroups = (nact + kGroup - 1) / kGroup;
+    unsigned* from = reinterpret_cast<unsigned*>(acc);
+    unsigned* to = from + 4 * npass;
+    for (int e = tid; e < slots; e += T) {
+      const unsigned m = mask[e >> 5];
+      if (!(m >> lane & 1)) continue;
+      int at = __popc(m & lt);
+      for (int k = 0; k < (e >> 5); k++) at += __popc(mask[k]);
+      const int4 q = __ldg(a.pos4 + sbase + e);
+      from[at] = order_key(q.x, org[0], C, e);
+      from[npass + at] = order_key(q.y, org[1], C, e);
+      from[2 * npass + at] = order_key(q.z, org[2], C, e);
+    }
+    // ... and ordered into compact groups: every range of more than one group
+    // is cut at the middle group along x, y, z in turn, each sink's place
+    // being its range's start plus the number of smaller keys in the range
+    // (keys are unique).  Groups of 8 keep 2.2 candidates per pair inside the
+    // cutoff at 64 sinks per cell (1.8 at 184), Morton order 2.5 (2.1).
+    if (!WRAP && ck != 0.f) {
+      const int pad = (ngroups * kGroup) - nact;  // the last group's absent sinks sort last
+      if (tid < pad) from[nact + tid] = from[npass + nact + tid] = from[2 * npass + nact + tid] = 0xffffffffu;
+      __syncthreads();
+      for (int level = 0; (1 << level) < ngroups; level++) {
+        const unsigned* axis = from + (level % 3) * npass;
+        for (int e = tid; e < nact; e += T) {
+          int lo = 0, hi = ngroups;  // the range of groups this position is in
+          for (int k = 0; k < level; k++) {
+            const int mid = lo + (hi - lo + 1) / 2;
+            if (hi - lo > 1) {
+              if ((e >> 3) < mid) hi = mid;
+              else lo = mid;
             }
           }
+          const unsigned m = axis[e];
+          int rank = lo * kGroup;
+          if (hi - lo > 1) {
+            for (int j = lo * kGroup; j < hi * kGroup; j += 4) {
+              const uint4 o = *reinterpret_cast<const uint4*>(axis + j);
+              rank += (o.x < m) + (o.y < m) + (o.z < m) + (o.w < m);
+            }
+          } else {
+            rank = e;
+          }
+          to[rank] = from[e];
+          to[npass + rank] = from[npass + e];
+          to[2 * npass + rank] = from[2 * npass + e];
         }
+        if (tid < pad) to[nact + tid] = to[npass + nact + tid] = to[2 * npass + nact + tid] = 0xffffffffu;
         __syncthreads();
+        unsigned* t = from;
+        from = to;
+        to = t;
       }
-    }
-    for (int e = tid; e < np; e += T) {
-      const unsigned m = skey[e];
-      const bool act = (m >> 8) < 512u;
-      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (act) {
-        const int4 q = __ldg(a.pos4 + sbase + (int32_t)(m & 0xffu));
-        p = make_float4(offset_scaled((uint32_t)q.x, ox, sc), offset_scaled((uint32_t)q.y, oy, sc),
-                        offset_scaled((uint32_t)q.z, oz, sc), 0.f);
-      }
-      spos[e] = p;
-#pragma unroll
-      for (int c = 0; c < 8; c++) acc[e * 8 + c] = 0.f;
-      // active sinks sort first: the first inactive slot is their count
-      if (!act && (e == 0 || (skey[e - 1] >> 8) < 512u)) runp[kMaxRuns + 1] = e;
-    }
-    __syncthreads();
-    const int nact = runp[kMaxRuns + 1];
-    const int ngroups = (nact + kGroup - 1) / kGroup;
-    int r = 0;  // this thread's neighbourhood run: its staged indices only increase
-    for (int c0 = 0; c0 < total; c0 += stage) {
-      const int len = min(stage, total - c0);
+    } else {
       __syncthreads();
+    }
+    for (int e = tid; e < nact; e += T) sidx[e] = (unsigned char)(from[e] & 0xffu);
+    __syncthreads();  // the keys' space becomes the sums'
+    for (int e = tid; e < nact; e += T) {
+      const int4 q = __ldg(a.pos4 + sbase + sidx[e]);
+      spos[e] = make_float4(offset_scaled((uint32_t)q.x, org[0], a.lscale), offset_scaled((uint32_t)q.y, org[1], a.lscale),
+                            offset_scaled((uint32_t)q.z, org[2], a.lscale), 0.f);
+      float4* A = reinterpret_cast<float4*>(acc + e * 8);
+      A[0] = A[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int c0 = 0; c0 < runp[kMaxRuns]; c0 += stage) {
+      const int len = min(stage, runp[kMaxRuns] - c0);
+      __syncthreads();
+      int r = 0;  // this thread's neighbourhood run: its staged indices only increase
       for (int j = tid; j < len; j += T) {
         const int e = c0 + j;
         while (runp[r + 1] <= e) r++;
         const int4 u = __ldg(a.pos4 + runb[r] + (e - runp[r]));
-        src[j] = make_float4(offset_scaled((uint32_t)u.x, ox, sc), offset_scaled((uint32_t)u.y, oy, sc),
-                             offset_scaled((uint32_t)u.z, oz, sc), 0.f);
+        src[j] = offset_scaled((uint32_t)u.x, org[0], a.lscale);
+        src[stage + j] = offset_scaled((uint32_t)u.y, org[1], a.lscale);
+        src[2 * stage + j] = offset_scaled((uint32_t)u.z, org[2], a.lscale);
       }
+      // the last step of 64 reads up to 63 entries past the chunk's end
+      for (int j = len + tid; j < ((len + 63) & ~63); j += T) src[j] = src[stage + j] = src[2 * stage + j] = kFar;
       __syncthreads();
       for (int g = warp; g < ngroups; g += W) {
         const int gs = g * kGroup;
         const int gn = min(kGroup, nact - gs);
         const bool mysink = t8 < gn;
+        // lanes without a sink (a partial group) hold a copy of the group's
+        // first sink; their sums are never committed
         const float4 sp = spos[gs + (mysink ? t8 : 0)];
         // group bounding box (lanes 0..gn-1 hold the sinks)
         float bxl = mysink ? sp.x : INFINITY, bxh = mysink ? sp.x : -INFINITY;
@@ -638,63 +697,97 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
           bzl = fminf(bzl, __shfl_xor_sync(0xffffffffu, bzl, o));
           bzh = fmaxf(bzh, __shfl_xor_sync(0xffffffffu, bzh, o));
         }
-        // box as centre and half-extent: the distance along an axis is then
-        // |s - c| - h (3 instructions instead of 4).  The half-extent is
-        // widened by 1e-5 of the unit (2 r_s; offsets here are a few units,
-        // whose float spacing is < 1e-6) to cover the rounding of c, h and
-        // s - c, so the cull never drops a source the exact pair test keeps.
-        const float cbx = 0.5f * (bxl + bxh), hbx = fmaf(0.5f, bxh - bxl, 1e-5f);
-        const float cby = 0.5f * (byl + byh), hby = fmaf(0.5f, byh - byl, 1e-5f);
-        const float cbz = 0.5f * (bzl + bzh), hbz = fmaf(0.5f, bzh - bzl, 1e-5f);
-        float px = 0.f, py = 0.f, pz = 0.f, pp = 0.f;
-        int cnt = 0;
-        // Every lane loads a staged source (the last one again past the end)
-        // and tests it; kept sources are appended to the warp's buffer.  The
-        // buffer is read only after a __syncwarp (flush or tail), so appends
-        // need no barrier of their own.
-        for (int j0 = 0; j0 < len; j0 += 32) {
-          const int j = j0 + lane;
-          const float4 s = src[min(j, len - 1)];
-          const float ex = fmaxf(fabsf(s.x - cbx) - hbx, 0.f);
-          const float ey = fmaxf(fabsf(s.y - cby) - hby, 0.f);
-          const float ez = fmaxf(fabsf(s.z - cbz) - hbz, 0.f);
-          const bool keep = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < keep2 && j < len;
-          const unsigned b = __ballot_sync(0xffffffffu, keep);
-          if (keep) buf[cnt + __popc(b & lt)] = s;
-          cnt += __popc(b);
+        // Box as centre and half-extent in cutoffs: the distance along an
+        // axis is |s - c| - h clamped to [0, 1] by the add's saturation (a
+        // distance of a cutoff or more is no candidate whatever the other
+        // axes are).  The half-extent is widened by cull_m to cover the
+        // rounding of c, h and s - c, so the cull never drops a source the
+        // exact pair test keeps.  Without a cutoff all scales are 0 and every
+        // source is kept.
+        const f32x2 k2 = pack2(ck, ck);
+        const float nx = -0.5f * (bxl + bxh) * ck, ny = -0.5f * (byl + byh) * ck, nz = -0.5f * (bzl + bzh) * ck;
+        const f32x2 ncx = pack2(nx, nx), ncy = pack2(ny, ny), ncz = pack2(nz, nz);
+        const float hx = fmaf(0.5f * ck, bxh - bxl, cm), hy = fmaf(0.5f * ck, byh - byl, cm),
+                    hz = fmaf(0.5f * ck, bzh - bzl, cm);
+        const f32x2 ns[3] = {pack2(-sp.x, -sp.x), pack2(-sp.y, -sp.y), pack2(-sp.z, -sp.z)};
+        f32x2 sum[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) sum[c] = pack2(0.f, 0.f);
+        int cnt = 0;   // buffered sources
+        int head = 0;  // ring position of the first of them: 0 or kFlush
+        // Every lane tests two staged sources; kept ones are appended to the
+        // warp's buffer.  The buffer is read only after a __syncwarp (flush
+        // or tail), so appends need no barrier of their own.
+        for (int j0 = 0; j0 < len; j0 += 64) {
+          const int j = j0 + 2 * lane;
+          const f32x2 sx = *reinterpret_cast<const f32x2*>(src + j);
+          const f32x2 sy = *reinterpret_cast<const f32x2*>(src + stage + j);
+          const f32x2 sz = *reinterpret_cast<const f32x2*>(src + 2 * stage + j);
+          const float2 dx = unpack2(fma2(sx, k2, ncx)), dy = unpack2(fma2(sy, k2, ncy)), dz = unpack2(fma2(sz, k2, ncz));
+          const f32x2 ex = pack2(__saturatef(fabsf(dx.x) - hx), __saturatef(fabsf(dx.y) - hx));
+          const f32x2 ey = pack2(__saturatef(fabsf(dy.x) - hy), __saturatef(fabsf(dy.y) - hy));
+          const f32x2 ez = pack2(__saturatef(fabsf(dz.x) - hz), __saturatef(fabsf(dz.y) - hz));
+          const float2 d2 = unpack2(fma2(ex, ex, fma2(ey, ey, mul2(ez, ez))));
+          bool k0 = d2.x < 1.0f, k1 = d2.y < 1.0f;
+          if (WRAP) {  // no far padding under the minimum image
+            k0 = k0 && j < len;
+            k1 = k1 && j + 1 < len;
+          }
+          const unsigned b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
+          const int at = head + cnt + __popc(b0 & lt) + __popc(b1 & lt);
+          const float2 x = unpack2(sx), y = unpack2(sy), z = unpack2(sz);
+          if (k0) {
+            float* p = buf + (at & (kBuf - 1));
+            p[0] = x.x;
+            p[kBuf] = y.x;
+            p[2 * kBuf] = z.x;
+          }
+          if (k1) {
+            float* p = buf + ((at + (k0 ? 1 : 0)) & (kBuf - 1));
+            p[0] = x.y;
+            p[kBuf] = y.y;
+            p[2 * kBuf] = z.y;
+          }
+          cnt += __popc(b0) + __popc(b1);
           // the count is the same in every lane; a vote makes the branch
           // warp-uniform for the compiler (no reconvergence region)
-          if (__all_sync(0xffffffffu, cnt >= 32)) {
+          if (__all_sync(0xffffffffu, cnt >= kFlush)) {
             __syncwarp();
-#pragma unroll
-            for (int k = 0; k < 32; k += 8) {
-              // lanes without a sink (a partial group) hold a copy of the
-              // group's first sink; their sums are never committed
-              pair2<WRAP>(pk, sp, buf[k + ph], buf[k + 4 + ph], px, py, pz, pp);
+#pragma unroll 1
+            for (int t = 0; t < kFlush; t += 16) {
+              const float* p = buf + head + t + 4 * ph;
+              const ulonglong2 ux = *reinterpret_cast<const ulonglong2*>(p);
+              const ulonglong2 uy = *reinterpret_cast<const ulonglong2*>(p + kBuf);
+              const ulonglong2 uz = *reinterpret_cast<const ulonglong2*>(p + 2 * kBuf);
+              const f32x2 u[3][2] = {{{ux.x}, {ux.y}}, {{uy.x}, {uy.y}}, {{uz.x}, {uz.y}}};
+              pairs<WRAP, 2>(pk, ns, u, sum, 4);
             }
-            __syncwarp();
-            if (lane < cnt - 32) buf[lane] = buf[32 + lane];
-            cnt -= 32;
+            cnt -= kFlush;
+            head ^= kFlush;
             __syncwarp();
           }
         }
+        // the rest, 8 sources a step: padded with far ones (under the
+        // minimum image with zeros that count excludes)
+        if (lane < ((8 - (cnt & 7)) & 7)) {
+          float* p = buf + ((head + cnt + lane) & (kBuf - 1));
+          p[0] = p[kBuf] = p[2 * kBuf] = WRAP ? 0.f : kFar;
+        }
         __syncwarp();
-        if (WRAP) {
-          for (int k = 0; k < cnt; k += 4) {
-            if (k + ph < cnt && mysink) {
-              const float4 u = buf[k + ph];
-              pair<WRAP>(pk, sp.x - u.x, sp.y - u.y, sp.z - u.z, px, py, pz, pp);
-            }
-          }
-        } else {
-          // past the count a lane takes a source 1e18 units away: beyond any
-          // cutoff, its terms are exactly 0 (no minimum-image fold here)
-          const float4 far = make_float4(1e18f, 1e18f, 1e18f, 0.f);
-          for (int k = 0; k < cnt; k += 8) {
-            const float4 u0 = k + ph < cnt ? buf[k + ph] : far;
-            const float4 u1 = k + 4 + ph < cnt ? buf[k + 4 + ph] : far;
-            pair2<WRAP>(pk, sp, u0, u1, px, py, pz, pp);
-          }
+        for (int t = 0; t < cnt; t += 8) {
+          const float* p = buf + head + t + 2 * ph;
+          const f32x2 u[3][1] = {{*reinterpret_cast<const f32x2*>(p)},
+                                 {*reinterpret_cast<const f32x2*>(p + kBuf)},
+                                 {*reinterpret_cast<const f32x2*>(p + 2 * kBuf)}};
+          pairs<WRAP, 1>(pk, ns, u, sum, cnt - t - 2 * ph);
+        }
+        float px, py, pz, pp;
+        {
+          const float2 vx = unpack2(sum[0]), vy = unpack2(sum[1]), vz = unpack2(sum[2]), vp = unpack2(sum[3]);
+          px = vx.x + vx.y;
+          py = vy.x + vy.y;
+          pz = vz.x + vz.y;
+          pp = -(vp.x + vp.y);
         }
         __syncwarp();
         // fold the four source phases (fixed order), lanes 0..7 hold the group's sums
@@ -724,7 +817,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
     __syncthreads();
     // 2. long-range interpolation and the kick, one thread per sorted sink
     for (int e = tid; e < nact; e += T) {
-      const int32_t i = sbase + (int32_t)(skey[e] & 0xffu);
+      const int32_t i = sbase + (int32_t)sidx[e];
       const float lx = a.gx[i], ly = a.gy[i], lz = a.gz[i], lp = a.pot[i];  // from k_interp_long
       const float* A = acc + e * 8;
       // pair sums back from units of 2 r_s: force x (1/2r_s)^2, potential x 1/2r_s
@@ -815,17 +908,19 @@ __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
     k_kick_batch(const KickArgs* __restrict__ boxes, KickArgs one, const int4* __restrict__ items,
                  const int* __restrict__ nitems, int* __restrict__ counter, StepScalars st, int stage, int npass) {
   extern __shared__ float4 smem4[];
-  __shared__ int s_item[2];
+  __shared__ int s_item[3];  // this and the next item, the number of items
   // The box's arguments are read from shared memory where they are used:
   // held in registers, its ten array addresses would spill the pair loop.
   __shared__ KickArgs s_args;
-  const int n = *nitems;
-  if (threadIdx.x == 0) s_item[0] = atomicAdd(counter, 1);
+  if (threadIdx.x == 0) {
+    s_item[0] = atomicAdd(counter, 1);
+    s_item[2] = *nitems;
+  }
   __syncthreads();
   int cur_box = -1;
   for (int k = 0;; k ^= 1) {
     const int it = s_item[k];
-    if (it >= n) return;
+    if (it >= s_item[2]) return;
     // the next item is fetched while this one runs; the barrier at the end of
     // the iteration orders the write against the reads of s_item[k ^ 1]
     if (threadIdx.x == 0) s_item[k ^ 1] = atomicAdd(counter, 1);
@@ -1056,12 +1151,16 @@ KickArgs make_args(tpm_ctx* c, const int b[3], const int e[3], int min_rung, dou
   a.h2 = (float)((c->opt.hsoft * su) * (c->opt.hsoft * su));
   a.rcut2 = c->rcut_box > 0 ? (float)((c->rcut_box * su) * (c->rcut_box * su)) : INFINITY;
   a.wlen = (float)su;
+  // The cull's distances in cutoffs: its rounding is below 4 float spacings
+  // of the largest offset from a cell's centre, 1.5 cells.
+  a.cull_k = c->rcut_box > 0 ? (float)(1.0 / (c->rcut_box * su)) : 0.0f;
+  a.cull_m = c->rcut_box > 0 ? (float)std::max(3e-6, 5e-7 * 1.5 / (c->C * c->rcut_box)) : 0.0f;
   return a;
 }
 
 size_t kick_smem(const KickShape& k) {
-  return sizeof(float4) * ((size_t)k.stage + (size_t)k.warps * kBuf + k.npass) + sizeof(float) * k.npass * 8 +
-         sizeof(unsigned) * k.npass + sizeof(int) * (2 * kMaxRuns + 2);
+  return sizeof(float) * 3 * ((size_t)k.stage + (size_t)k.warps * kBuf) + sizeof(float4) * k.npass +
+         sizeof(float) * k.npass * 8 + k.npass + sizeof(int) * (2 * kMaxRuns + 1 + kPass / 32 + 6);
 }
 
 }  // namespace
