@@ -62,8 +62,9 @@ int64_t plan_bytes(const tpm_options& o, int64_t cap) {
   b += cap * 16;                               // pos4
   b += cap * 4 * 5 + 8;                        // key, idx, cellof, prefix, slot
   const int64_t T = kScanTileElems;
-  b += 4 * (2 * ((cap + T - 1) / T + (ncell + T - 1) / T) + 64);  // blocksums
-  b += 8 * ((std::max(cap, ncell) + T - 1) / T + 1);  // look-back status words
+  b += 4 * (kBlocksumPerTile * ((std::max(cap, ncell) + T - 1) / T) + 64);  // block sums, node heads
+  b += 8 * ((std::max(cap, ncell) + T - 1) / T + 1) + 4 * kSortCounters;  // look-back status words, counters
+  b += 4 * unit_cuts_entries((int)C);          // partition unit intervals
   b += 8 * (ncell + 2);                        // counts + offsets
   b += N * N * N * 4 * 2 + N * N * (int64_t)fft3d_padded_columns((int)N) * 8 + 3 * N * 8;  // rho, phi, rhok, twiddles
   return b;
@@ -256,6 +257,18 @@ struct ScratchField {
   int64_t count;
 };
 
+// Entries of each of the four arrays in sort4: 16-byte aligned.
+int64_t sort4_stride(int64_t cap) { return (cap + 3) / 4 * 4; }
+
+// The arrays inside sort4, once it is allocated or bound.
+void carve_sort4(tpm_ctx* c) {
+  const int64_t n = sort4_stride(std::max<int64_t>(c->cap, 1));
+  c->key = static_cast<uint32_t*>(c->sort4);
+  c->idx = c->sort4 ? reinterpret_cast<int32_t*>(c->key) + n : nullptr;
+  c->cellof = c->sort4 ? c->idx + n : nullptr;
+  c->slot = c->sort4 ? c->cellof + n : nullptr;
+}
+
 std::vector<ScratchField> scratch_fields(tpm_ctx* c) {
   const int64_t cap = std::max<int64_t>(c->cap, 1);
   const int64_t N = c->N, C = c->C, ncell = C * C * C;
@@ -265,8 +278,7 @@ std::vector<ScratchField> scratch_fields(tpm_ctx* c) {
       {(void**)&c->pot, 4, cap},     {(void**)&c->pos4, 16, cap},    {(void**)&c->x2, 4, cap},
       {(void**)&c->y2, 4, cap},      {(void**)&c->z2, 4, cap},       {(void**)&c->vx2, 4, cap},
       {(void**)&c->vy2, 4, cap},     {(void**)&c->vz2, 4, cap},      {(void**)&c->rung2, 1, cap},
-      {(void**)&c->key, 4, cap},     {(void**)&c->idx, 4, cap},      {(void**)&c->cellof, 4, cap},
-      {(void**)&c->prefix, 4, cap + 1}, {(void**)&c->slot, 4, cap},  {(void**)&c->blocksum, 4, 2 * nb + 64},
+      {(void**)&c->sort4, 16, sort4_stride(cap)}, {(void**)&c->prefix, 4, cap + 1}, {(void**)&c->blocksum, 4, kBlocksumPerTile * nb + 64},
       {(void**)&c->rho, 4, N * N * N}, {(void**)&c->rhok, 8, N * N * fft3d_padded_columns((int)N)},
       {(void**)&c->phi, 4, N * N * N},
   };
@@ -287,6 +299,7 @@ void ctx_bind_scratch(tpm_ctx* c, void* base, cudaStream_t s) {
     *f.ptr = p;
     p += (f.elem * f.count + kScratchAlign - 1) / kScratchAlign * kScratchAlign;
   }
+  carve_sort4(c);
   c->stream = s;
   if (c->plans) {
     cufftSetStream(c->plan_r2c, s);
@@ -296,6 +309,7 @@ void ctx_bind_scratch(tpm_ctx* c, void* base, cudaStream_t s) {
 
 void ctx_unbind_scratch(tpm_ctx* c, cudaStream_t own) {
   for (const ScratchField& f : scratch_fields(c)) *f.ptr = nullptr;
+  carve_sort4(c);
   c->stream = own;
   if (c->plans) {
     cufftSetStream(c->plan_r2c, own);
@@ -350,12 +364,13 @@ int tpm::ctx_create(const tpm_options* opts, int64_t capacity, bool with_scratch
   A.get(c->vy, capacity);
   A.get(c->vz, capacity);
   A.get(c->rung, capacity);
-  A.get(c->scan_status, nb + 1);
+  A.get(c->scan_status, nb + 1 + kSortCounters / 2);
   A.get(c->cell_count, ncell + 1);
   A.get(c->cell_begin, ncell + 1);
   A.get(c->thr, C + 1);
   A.get(c->tree, C * kMaxTreeDepth);
   A.get(c->depth1d, C);
+  A.get(c->unit_cuts, unit_cuts_entries((int)C));
   A.get(c->fft_tw, 3 * N);
   A.get(c->gtab, 2 * N);
   A.get(c->k2tab, N);
@@ -378,8 +393,9 @@ int tpm::ctx_create(const tpm_options* opts, int64_t capacity, bool with_scratch
     tpm_ctx_destroy(c);
     return A.status;
   }
+  if (with_scratch) carve_sort4(c);
   e = cudaMemset(c->d_err, 0, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(c->scan_status, 0, sizeof(unsigned long long) * (nb + 1));
+  if (e == cudaSuccess) e = cudaMemset(c->scan_status, 0, sizeof(unsigned long long) * (nb + 1 + kSortCounters / 2));
   if (e == cudaSuccess) e = cudaMemset(c->cell_begin, 0, sizeof(int32_t) * (ncell + 1));
   if (e != cudaSuccess) {
     tpm_ctx_destroy(c);
@@ -401,7 +417,7 @@ int tpm_ctx_destroy(tpm_ctx* c) {
   if (!c) return TPM_OK;
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* ptrs[] = {c->x, c->y, c->z, c->vx, c->vy, c->vz, c->rung, c->scan_status, c->cell_count, c->cell_begin,
-                  c->thr, c->tree, c->depth1d, c->fft_tw, c->gtab, c->k2tab, c->d_err};
+                  c->thr, c->tree, c->depth1d, c->unit_cuts, c->fft_tw, c->gtab, c->k2tab, c->d_err};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   void* kq[] = {c->kq.d_args, c->kq.d_cells, c->kq.d_class, c->kq.d_hist, c->kq.d_items, c->kq.d_nitems,

@@ -19,6 +19,8 @@ constexpr int kPhiBW = 3;         // PHI_BW, tigerpm/tigerpm.hpp:41
 // look-back status words allocated with the context (chainmesh.cu checks
 // that its scan kernels use the same tile).
 constexpr int kScanTileElems = 4096;
+// ints of the block-sum array per tile: two sums, or four 16-byte node heads
+constexpr int kBlocksumPerTile = 16;
 constexpr int kMaxTreeDepth = 24; // 1-D bisection depth bound (C < 2^23)
 constexpr int kDepositFracBits = 40;
 
@@ -41,6 +43,21 @@ int fail(int status, const std::string& msg);
     if (r_ != CUFFT_SUCCESS)                                                     \
       return ::tpm::fail(TPM_ERR_CUFFT, std::string(#call) + " failed: " + std::to_string((int)r_)); \
   } while (0)
+
+// Counters of one sort behind its look-back words: a tile counter per
+// partition level (at most 3 x 12), the number of large units, the jumps of
+// the final order.
+constexpr int kSortCounters = 64, kSortBig = 62, kSortJumps = 63;
+
+// Intervals of the 1-D bisection at one depth: their place among the context's
+// unit_cuts, their number and the widest one.
+struct UnitLevel {
+  int at = 0, count = 0;
+  int64_t widest = 0;
+};
+// Entries of unit_cuts: every depth's interval starts and the end, chain_dim
+// at most 2048 (12 depths).
+inline int64_t unit_cuts_entries(int C) { return 12 * ((int64_t)C + 1); }
 
 // One node of the 1-D bisection tree over [0, C) that the reference's chain
 // sort applies per dimension (split at lo + span/2, src/chainmesh.cpp:198).
@@ -100,20 +117,22 @@ struct tpm_ctx {
   uint32_t *x2 = nullptr, *y2 = nullptr, *z2 = nullptr;
   float *vx2 = nullptr, *vy2 = nullptr, *vz2 = nullptr;
   int8_t* rung2 = nullptr;
+  void* sort4 = nullptr;      // key, idx, cellof and slot, one block of 16 bytes per particle
   uint32_t* key = nullptr;    // cell key of the particle at each position
   int32_t* idx = nullptr;     // original index of the particle at each position
   int32_t* cellof = nullptr;  // final cell whose range holds each position
-  int32_t* prefix = nullptr;  // exclusive scan of the per-level flags (n + 1)
-  int32_t* slot = nullptr;    // partner positions of right-misplaced elements
-  int32_t* blocksum = nullptr;
-  unsigned long long* scan_status = nullptr;  // look-back words, one per scan tile
+  int32_t* prefix = nullptr;  // misplaced elements of each node of a level, then the final order (n + 1)
+  int32_t* slot = nullptr;    // positions of a level's misplaced elements
+  int32_t* blocksum = nullptr;  // tile sums of the cell counts, then node heads of a partition level
+  unsigned long long* scan_status = nullptr;  // look-back words, one per scan tile, then kSortCounters ints
   int32_t* cell_count = nullptr;
   int32_t* cell_begin = nullptr;  // C^3 + 1
   uint32_t* thr = nullptr;        // per-dim split thresholds, C + 1
   tpm::TreeNode* tree = nullptr;  // [C * kMaxTreeDepth]
   int* depth1d = nullptr;         // [C]
   int max_depth1d = 0;
-  uint64_t scan_stamp = 0;  // distinguishes look-back status words of successive scans
+  int* unit_cuts = nullptr;                  // interval starts of every bisection depth (sort_init)
+  std::vector<tpm::UnitLevel> unit_levels;   // one per depth
 
   // mesh
   float* rho = nullptr;  // N^3 real grid (deposit out, r2c in)
