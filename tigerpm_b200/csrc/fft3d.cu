@@ -531,14 +531,22 @@ constexpr LinePlan reverse_plan(const LinePlan& p) {
   return q;
 }
 
+// Columns of the half spectrum of a mesh of N: N/2 + 1 rounded up to kLineCols.
+constexpr int padded_columns(int N) { return ((N / 2 + 1) + kLineCols - 1) / kLineCols * kLineCols; }
+
 template <int N>
 struct LineCfg {
   static constexpr LinePlan P = line_plan(N);
+  static constexpr int Sz = padded_columns(N);
   static constexpr int TL = P.TL, E = P.E;
   static constexpr int kThreads = kLineCols * TL;
-  // line stride = N + 4 (N % 16 == 0): the transposed column loads of 8
-  // columns x 4 rows per warp then fall in distinct bank pairs
+  // Line stride of the z passes (a line's lanes are neighbours in a warp) and
+  // of the column passes (a warp is 8 lines x 4 lanes): with N % 16 == 0 the
+  // latter puts the 8 lines 4 banks apart, so that 16 threads' 8-byte accesses
+  // (8 lines x 2 lanes) and 8 threads' 16-byte ones (8 lines) meet no bank
+  // twice, whatever the stride between lanes.
   static constexpr int LS = N + 4;
+  static constexpr int LSC = N + 2;
   // resident threads per SM the register budget targets: 768 (85 registers),
   // 512 (128 registers) from 28 values per lane up
   static constexpr int kMinBlocks = (E >= 28 ? 2 : 3) * 256 / kThreads;
@@ -549,16 +557,25 @@ struct LineCfg {
   static constexpr size_t kSmem = sizeof(float2) * ((size_t)N + (size_t)kLineCols * LS);
   // the x pass holds the stage tables of both radix orders and the x axis's
   // Green's-function and k^2 tables (read from shared memory, not L1)
-  static constexpr size_t kSmemX = kSmem + sizeof(float2) * (size_t)N + sizeof(float) * 2 * (size_t)N;
-  static_assert(P.ns >= 1 && P.ns <= 6, "no line plan for this N");
+  static constexpr size_t kSmemX =
+      sizeof(float2) * (2 * (size_t)N + (size_t)kLineCols * LSC) + sizeof(float) * 2 * (size_t)N;
+  static constexpr size_t kSmemC = sizeof(float2) * ((size_t)N + (size_t)kLineCols * LSC);
+  static_assert(P.ns >= 2 && P.ns <= 6, "no line plan for this N");
 };
 
 // One line transform of sign S with the plan of N (REV: its radices reversed).
-template <int N, int S, bool REV = false>
+// COL: the lines' threads are spread over the block's warps (column passes),
+// so the exchanges between stages are block barriers.
+template <int N, int S, bool REV = false, bool COL = false>
 struct LineFft {
   using L = LineCfg<N>;
   static constexpr LinePlan P = REV ? reverse_plan(L::P) : L::P;
   static constexpr int TL = L::TL, E = L::E;
+
+  __device__ __forceinline__ static void sync() {
+    if (COL) __syncthreads();
+    else __syncwarp();
+  }
 
   // Stage ST: v holds its inputs, v[b R + r] = x[j + r N / R] for the lane's
   // butterflies j = lane + TL b; twiddles exp(S 2 pi i (j mod Ns) r / (Ns R))
@@ -612,13 +629,13 @@ struct LineFft {
           for (int r = 0; r < R; r++) line[q * NS * R + k + r * NS] = v[b * R + r];
         }
       }
-      __syncwarp();
+      sync();
       constexpr int R2 = P.rad[ST + 1];
 #pragma unroll
       for (int b = 0; b < E / R2; b++)
 #pragma unroll
         for (int r = 0; r < R2; r++) v[b * R2 + r] = line[lane + TL * b + r * (N / R2)];
-      __syncwarp();
+      sync();
       stage<ST + 1>(line, v, tw, lane, out);
     }
   }
@@ -657,47 +674,6 @@ struct LineFft {
 template <int N>
 __device__ __forceinline__ void line_twiddles(float2* s_tw, const float2* __restrict__ tw) {
   for (int i = threadIdx.x; i < N; i += LineCfg<N>::kThreads) s_tw[i] = __ldg(tw + i);
-}
-
-// Load / store the block's kLineCols columns (rows y < N at stride rs) into /
-// from the transposed shared-memory lines, two columns per 16-byte access.
-// Every load is issued before the first shared store (E / 2 loads in flight
-// per thread).
-template <int N>
-__device__ __forceinline__ void cols_load(float2* __restrict__ lines, const float2* __restrict__ g, int64_t rs) {
-  using L = LineCfg<N>;
-  constexpr int IT = (kLineCols / 2) * N / L::kThreads;
-  static_assert(IT * L::kThreads == (kLineCols / 2) * N, "column tile per thread");
-  float4 u[IT];
-#pragma unroll
-  for (int i = 0; i < IT; i++) {
-    const int e = threadIdx.x + i * L::kThreads;
-    const int y = e / (kLineCols / 2), c = 2 * (e - y * (kLineCols / 2));
-    u[i] = __ldg(reinterpret_cast<const float4*>(g + y * rs + c));
-  }
-#pragma unroll
-  for (int i = 0; i < IT; i++) {
-    const int e = threadIdx.x + i * L::kThreads;
-    const int y = e / (kLineCols / 2), c = 2 * (e - y * (kLineCols / 2));
-    lines[c * L::LS + y] = make_float2(u[i].x, u[i].y);
-    lines[(c + 1) * L::LS + y] = make_float2(u[i].z, u[i].w);
-  }
-}
-template <int N>
-__device__ __forceinline__ void cols_store(const float2* __restrict__ lines, float2* __restrict__ g, int64_t rs) {
-  using L = LineCfg<N>;
-  constexpr int IT = (kLineCols / 2) * N / L::kThreads;
-  // thread index through an opaque move: the load's address arithmetic is
-  // then recomputed here instead of being kept live across the transform
-  int t;
-  asm volatile("mov.b32 %0, %1;" : "=r"(t) : "r"((int)threadIdx.x));
-#pragma unroll
-  for (int i = 0; i < IT; i++) {
-    const int e = t + i * L::kThreads;
-    const int y = e / (kLineCols / 2), c = 2 * (e - y * (kLineCols / 2));
-    const float2 a = lines[c * L::LS + y], b = lines[(c + 1) * L::LS + y];
-    *reinterpret_cast<float4*>(g + y * rs + c) = make_float4(a.x, a.y, b.x, b.y);
-  }
 }
 
 // P1 (line engine): rows (x, 2p), (x, 2p+1) as one complex line, forward z
@@ -739,69 +715,74 @@ __global__ void __launch_bounds__(LineCfg<N>::kThreads, LineCfg<N>::kMinBlocks)
   }
 }
 
-// P2 / P4 (line engine): the 8 columns [c0, c0 + 8) of plane x along y.
+// P2 / P4 (line engine): the 8 columns [c0, c0 + 8) of plane x along y.  A
+// thread's line is its column and neighbouring threads have neighbouring
+// columns, so the first stage's inputs come straight from global memory and
+// the last stage's outputs go straight back, 64 contiguous bytes per row.
+// The passes were bound by shared-memory wavefronts (89 % of the pipe): the
+// columns were staged there both ways, and with a line's lanes side by side in
+// a warp the stages' stores met 2-way bank conflicts and every lane its own
+// twiddle; now a twiddle read serves 8 lines and only the exchanges are left.
+// 384^3: y passes 139 -> 92 us (0.69 of the copy bandwidth), x pass 257 -> 188
+// us; 768^3: forward z + y 1.81 -> 1.49 ms, x 2.06 -> 1.65, inverse 1.92 -> 1.59.
 template <int N, int S>
 __global__ void __launch_bounds__(LineCfg<N>::kThreads, LineCfg<N>::kMinBlocks)
-    k_line_y(float2* __restrict__ Y, int Sz, const float2* __restrict__ tw, int x0) {
+    k_line_y(float2* __restrict__ Y, const float2* __restrict__ tw) {
   using L = LineCfg<N>;
+  using F = LineFft<N, S, false, true>;
   extern __shared__ __align__(16) float2 lsm[];
   float2* s_tw = lsm;
-  float2* lines = lsm + N;
   line_twiddles<N>(s_tw, tw);
-  const int li = threadIdx.x / L::TL, lane = threadIdx.x - li * L::TL;
-  float2* line = lines + li * L::LS;
-  const int per_x = Sz / kLineCols;
-  const int xb = blockIdx.x / per_x;
-  const int c0 = (blockIdx.x - xb * per_x) * kLineCols;
-  float2* plane = Y + (int64_t)(x0 + xb) * N * Sz + c0;
-  cols_load<N>(lines, plane, Sz);
-  __syncthreads();
-  LineFft<N, S>::run(
-      line, s_tw, lane, [&](int n) { return line[n]; }, [&](int n, float2 v) { line[n] = v; });
-  __syncthreads();
-  cols_store<N>(lines, plane, Sz);
+  const int li = threadIdx.x % kLineCols, lane = threadIdx.x / kLineCols;
+  float2* line = lsm + N + li * L::LSC;
+  constexpr int per_x = L::Sz / kLineCols;
+  const int x = blockIdx.x / per_x;
+  float2* col = Y + (int64_t)x * N * L::Sz + (blockIdx.x - x * per_x) * kLineCols + li;
+  float2 v[L::E];
+  F::load(v, lane, [&](int n) { return col[n * L::Sz]; });
+  __syncthreads();  // twiddles
+  F::from_regs(line, v, s_tw, lane, [&](int n, float2 u) { col[n * L::Sz] = u; });
 }
 
-// P3 (line engine): the 8 columns [c0, c0 + 8) of row y along x: forward
-// transform, Green's function (as k_fft_x_green), inverse transform.  The
-// inverse runs the reversed radix plan, so it starts from the registers the
-// forward transform ends in, with the Green's function applied there: the
-// spectrum of the line does not go through shared memory between the two.
+// P3 (line engine): the 8 columns [c0, c0 + 8) of row y along x, laid out as in
+// the y passes: forward transform, Green's function (as k_fft_x_green),
+// inverse transform.  The inverse runs the reversed radix plan, so it starts
+// from the registers the forward transform ends in, with the Green's function
+// applied there: the spectrum of the line does not go through shared memory
+// between the two.
 // tw: the forward plan's stage tables, then the reversed plan's (N each).
 template <int N>
 __global__ void __launch_bounds__(LineCfg<N>::kThreads, LineCfg<N>::kMinBlocksX)
-    k_line_x_green(float2* __restrict__ Y, int Sz, const float2* __restrict__ tw, const float* __restrict__ gt,
+    k_line_x_green(float2* __restrict__ Y, const float2* __restrict__ tw, const float* __restrict__ gt,
                    const float* __restrict__ k2tab, float norm) {
   using L = LineCfg<N>;
-  using Fwd = LineFft<N, -1, false>;
-  using Inv = LineFft<N, 1, true>;
+  using Fwd = LineFft<N, -1, false, true>;
+  using Inv = LineFft<N, 1, true, true>;
   extern __shared__ __align__(16) float2 lsm[];
   float2* s_tw = lsm;
   float2* s_twr = lsm + N;
   float2* lines = lsm + 2 * N;
+  const int li = threadIdx.x % kLineCols, lane = threadIdx.x / kLineCols;
+  float2* line = lines + li * L::LSC;
+  constexpr int per_y = L::Sz / kLineCols;
+  const int y = blockIdx.x / per_y;
+  const int c0 = (blockIdx.x - y * per_y) * kLineCols;
+  constexpr int64_t xs = (int64_t)N * L::Sz;
+  float2* col = Y + (int64_t)y * L::Sz + c0 + li;
+  float2 v[L::E];
+  Fwd::load(v, lane, [&](int n) { return col[n * xs]; });
   for (int i = threadIdx.x; i < 2 * N; i += L::kThreads) s_tw[i] = __ldg(tw + i);
-  float* s_gt = reinterpret_cast<float*>(lines + kLineCols * L::LS);
+  float* s_gt = reinterpret_cast<float*>(lines + kLineCols * L::LSC);
   float* s_k2 = s_gt + N;
   for (int i = threadIdx.x; i < N; i += L::kThreads) {
     s_gt[i] = __ldg(gt + i);
     s_k2[i] = __ldg(k2tab + i);
   }
-  const int li = threadIdx.x / L::TL, lane = threadIdx.x - li * L::TL;
-  float2* line = lines + li * L::LS;
-  const int per_y = Sz / kLineCols;
-  const int y = blockIdx.x / per_y;
-  const int c0 = (blockIdx.x - y * per_y) * kLineCols;
-  float2* col = Y + (int64_t)y * Sz + c0;
-  const int64_t xs = (int64_t)N * Sz;
-  cols_load<N>(lines, col, xs);
-  __syncthreads();
   const int kz = c0 + li;
   const bool live = kz < N / 2 + 1;
   const float k2yz = __ldg(k2tab + y) + (live ? __ldg(k2tab + kz) : 0.f);
   const float gyz = __ldg(gt + y) * (live ? __ldg(gt + kz) : 0.f);
-  float2 v[L::E];
-  Fwd::load(v, lane, [&](int n) { return line[n]; });
-  __syncwarp();
+  __syncthreads();
   Fwd::from_regs(line, v, s_tw, lane, [](int, float2) {});
   // v[b RL + r] = X[lane + TL b + r N / RL]: the Green's function in registers
   constexpr int RL = Fwd::P.rad[Fwd::P.ns - 1];
@@ -819,9 +800,7 @@ __global__ void __launch_bounds__(LineCfg<N>::kThreads, LineCfg<N>::kMinBlocksX)
   // live across the inverse (it would spill).
   int lane2;
   asm volatile("mov.b32 %0, %1;" : "=r"(lane2) : "r"(lane));
-  Inv::from_regs(line, v, s_twr, lane2, [&](int n, float2 u) { line[n] = u; });
-  __syncthreads();
-  cols_store<N>(lines, col, xs);
+  Inv::from_regs(line, v, s_twr, lane2, [&](int n, float2 u) { col[n * xs] = u; });
 }
 
 // P5 (line engine): spectrum rows 2p, 2p+1 recombined (Z = A + i B, the
@@ -875,8 +854,8 @@ int line_set_smem() {
   using L = LineCfg<N>;
   const int s = (int)L::kSmem;
   TPM_CUDA_TRY(cudaFuncSetAttribute(k_line_z_r2c<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
-  TPM_CUDA_TRY(cudaFuncSetAttribute(k_line_y<N, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
-  TPM_CUDA_TRY(cudaFuncSetAttribute(k_line_y<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
+  TPM_CUDA_TRY(cudaFuncSetAttribute(k_line_y<N, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmemC));
+  TPM_CUDA_TRY(cudaFuncSetAttribute(k_line_y<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmemC));
   TPM_CUDA_TRY(
       cudaFuncSetAttribute(k_line_x_green<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kSmemX));
   TPM_CUDA_TRY(cudaFuncSetAttribute(k_line_z_c2r<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, s));
@@ -895,13 +874,13 @@ int line_poisson(tpm_ctx* c, float2* Y, int Sz, const float* gt, float norm) {
   const float2* tw = c->fft_tw + N;  // the stage tables of the line plan, then of its reversal
   stage_begin(c, kStFftF);
   k_line_z_r2c<N><<<zblocks, L::kThreads, L::kSmem, s>>>(c->rho, Y, Sz, tw, 0);
-  k_line_y<N, -1><<<cblocks, L::kThreads, L::kSmem, s>>>(Y, Sz, tw, 0);
+  k_line_y<N, -1><<<cblocks, L::kThreads, L::kSmemC, s>>>(Y, tw);
   stage_end(c, kStFftF);
   stage_begin(c, kStGreen);
-  k_line_x_green<N><<<cblocks, L::kThreads, L::kSmemX, s>>>(Y, Sz, tw, gt, c->k2tab, norm);
+  k_line_x_green<N><<<cblocks, L::kThreads, L::kSmemX, s>>>(Y, tw, gt, c->k2tab, norm);
   stage_end(c, kStGreen);
   stage_begin(c, kStFftI);
-  k_line_y<N, 1><<<cblocks, L::kThreads, L::kSmem, s>>>(Y, Sz, tw, 0);
+  k_line_y<N, 1><<<cblocks, L::kThreads, L::kSmemC, s>>>(Y, tw);
   k_line_z_c2r<N><<<zblocks, L::kThreads, L::kSmem, s>>>(Y, c->phi, Sz, tw, 0);
   stage_end(c, kStFftI);
   c->launches += 5;
@@ -982,7 +961,7 @@ int plane_group(const tpm_ctx* c, int N) {
 
 }  // namespace
 
-int fft3d_padded_columns(int N) { return ((N / 2 + 1) + kLineCols - 1) / kLineCols * kLineCols; }
+int fft3d_padded_columns(int N) { return padded_columns(N); }
 
 bool fft3d_supported(int N) {
   FftPlan p;
