@@ -505,12 +505,20 @@ constexpr LinePlan line_plan_tl(int N, int TL) {
   return p;
 }
 
-// Fewest stages with at most 36 values per lane; ties go to more lanes per line.
+// Fewest stages with at most 36 values per lane; ties go to more lanes per
+// line.  Lanes are a power of two within a warp where such a plan exists;
+// else (400, 432, 720) a line's threads may straddle warps.
 constexpr LinePlan line_plan(int N) {
   LinePlan best{0, 0, 99, {1, 1, 1, 1, 1, 1}};
   constexpr int tls[4] = {32, 16, 8, 4};
   for (int i = 0; i < 4; i++) {
     const LinePlan p = line_plan_tl(N, tls[i]);
+    if (p.ns < 99 && p.E <= 36 && p.ns < best.ns) best = p;
+  }
+  if (best.ns < 99) return best;
+  constexpr int more[5] = {36, 24, 20, 18, 12};
+  for (int i = 0; i < 5; i++) {
+    const LinePlan p = line_plan_tl(N, more[i]);
     if (p.ns < 99 && p.E <= 36 && p.ns < best.ns) best = p;
   }
   return best;
@@ -540,6 +548,7 @@ struct LineCfg {
   static constexpr int Sz = padded_columns(N);
   static constexpr int TL = P.TL, E = P.E;
   static constexpr int kThreads = kLineCols * TL;
+  static constexpr bool kInWarp = (TL & (TL - 1)) == 0;  // a line's threads share a warp in the z passes
   // Line stride of the z passes (a line's lanes are neighbours in a warp) and
   // of the column passes (a warp is 8 lines x 4 lanes): with N % 16 == 0 the
   // latter puts the 8 lines 4 banks apart, so that 16 threads' 8-byte accesses
@@ -573,7 +582,7 @@ struct LineFft {
   static constexpr int TL = L::TL, E = L::E;
 
   __device__ __forceinline__ static void sync() {
-    if (COL) __syncthreads();
+    if (COL || !L::kInWarp) __syncthreads();
     else __syncwarp();
   }
 
@@ -666,7 +675,7 @@ struct LineFft {
                                              In in, Out out) {
     float2 v[E];
     load(v, lane, in);
-    __syncwarp();
+    sync();
     stage<0>(line, v, tw, lane, out);
   }
 };
@@ -698,7 +707,7 @@ __global__ void __launch_bounds__(LineCfg<N>::kThreads, LineCfg<N>::kMinBlocks)
   LineFft<N, -1>::run(
       line, s_tw, lane, [&](int n) { return make_float2(__ldg(r0 + n), __ldg(r1 + n)); },
       [&](int n, float2 v) { line[n] = v; });
-  __syncwarp();
+  LineFft<N, -1>::sync();
   float2* y0 = Y + row * Sz;
   float2* y1 = y0 + Sz;
   constexpr int Nh = N / 2 + 1;
@@ -891,7 +900,7 @@ int line_poisson(tpm_ctx* c, float2* Y, int Sz, const float* gt, float norm) {
 // Mesh sizes with a compiled line plan (the benchmark meshes, the batched
 // and served box meshes, and the powers of two up to 1024).
 #define TPM_LINE_SIZES(X) \
-  X(64) X(96) X(128) X(144) X(160) X(192) X(240) X(256) X(288) X(320) X(384) X(512) X(576) X(640) X(768) X(1024)
+  X(48) X(64) X(80) X(96) X(128) X(144) X(160) X(192) X(240) X(256) X(288) X(320) X(384) X(400) X(432) X(480) X(512) X(576) X(640) X(720) X(768) X(1024)
 
 bool line_supported(int N) {
   switch (N) {
