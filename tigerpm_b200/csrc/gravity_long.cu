@@ -141,12 +141,19 @@ static_assert(kDep32FracBits == 26 && kDepositFracBits == 40, "fixed-point scale
 // it: 9 to 16 rows of 3 to 4 x cells, up to twice 8x the tile's own) are one
 // flat index space over at most kDepRuns contiguous runs; each thread loads
 // kDepBatch candidates at a time (independent loads in flight), and the
-// reaching ones are compacted into a shared list of up to kDepList particle
+// reaching ones are compacted into a shared list of up to dep_list particle
 // indices before they are deposited, so that every thread of the block
 // deposits an equal share.
-constexpr int kDepThreads = 256;
+// The FP32 adds are latency-bound (shared compare-and-swap loops), so such a
+// block has 384 threads at 56 registers, three to an SM: 3.46 -> 2.98 ms at
+// 768^3 against 256 threads, 0.47 -> 0.40 ms at 384^3 (512 threads at 42
+// registers 3.36 ms, two blocks of 512 3.50 ms).  The integer adds, which
+// return at once, keep 256.
+template <int M>
+constexpr int dep_threads = M == kDepF32 ? 384 : 256;
+template <int M>
+constexpr int dep_list = 8 * dep_threads<M>;
 constexpr int kDepBatch = 4;
-constexpr int kDepList = 2048;
 constexpr int kDepRuns = 64;
 
 // Weights of one particle added to the tile (stencil origin o, extent ext);
@@ -190,7 +197,8 @@ __device__ __forceinline__ void deposit_particle(typename DepAcc<M>::T* acc, int
 }
 
 template <int T, int ASSIGN, int M>
-__global__ void __launch_bounds__(kDepThreads, 3) k_deposit(DepositArgs a) {
+__global__ void __launch_bounds__(dep_threads<M>, 3) k_deposit(DepositArgs a) {
+  constexpr int kDepThreads = dep_threads<M>, kDepList = dep_list<M>;
   constexpr int W = Width<ASSIGN>::W;
   extern __shared__ __align__(16) unsigned char dep_smem[];
   // the list follows the tile (a kDepF32 redo of a kDepI32 tile uses the
@@ -210,14 +218,16 @@ __global__ void __launch_bounds__(kDepThreads, 3) k_deposit(DepositArgs a) {
   const int o[3] = {tx * T, ty * T, tz * T};
   int ext[3];
   for (int d = 0; d < 3; d++) ext[d] = min(T, N - o[d]);
-  // chain cells whose particles can reach the tile: XN in [o-2, o+T+1)
-  int clo[3], cnt[3];
-  for (int d = 0; d < 3; d++) {
-    const int lo = (int)floor(((double)o[d] - 2.001) * C / N);
-    const int hi = (int)floor(((double)o[d] + T + 1.001) * C / N);
-    clo[d] = lo;
-    cnt[d] = min(hi - lo + 1, C);
-    if (cnt[d] == C) clo[d] = 0;
+  // chain cells whose particles can reach the tile: XN in [o-2, o+T+1); in
+  // shared memory, since held in registers they spill the candidate loop
+  __shared__ int s_clo[3], s_cnt[3];
+  if (threadIdx.x < 3) {
+    const int od = threadIdx.x == 0 ? o[0] : threadIdx.x == 1 ? o[1] : o[2];
+    const int lo = (int)floor(((double)od - 2.001) * C / N);
+    const int hi = (int)floor(((double)od + T + 1.001) * C / N);
+    const int n = min(hi - lo + 1, C);
+    s_clo[threadIdx.x] = n == C ? 0 : lo;
+    s_cnt[threadIdx.x] = n;
   }
   // The whole tile with accumulator mode MODE (its zeroing, the candidate
   // scan and the deposits); returns, for kDepI32, whether a point may have
@@ -250,21 +260,18 @@ __global__ void __launch_bounds__(kDepThreads, 3) k_deposit(DepositArgs a) {
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
   };
-  // x cells clo..clo+cnt-1 (mod C) of a (z, y) row: one or two contiguous runs
-  const int x0 = wrapi(clo[0], C);
-  const int xend = x0 + cnt[0];
-  const int nparts = xend > C ? 2 : 1;
-  const int nrows = cnt[2] * cnt[1];
   constexpr int kRowsPerBatch = kDepRuns / 2;
-  for (int row0 = 0; row0 < nrows; row0 += kRowsPerBatch) {
+  for (int row0 = 0; row0 < s_cnt[2] * s_cnt[1]; row0 += kRowsPerBatch) {
     // run table of rows [row0, row0 + kRowsPerBatch): run t = row t / 2,
     // part t % 2 (empty where the row or the part does not exist), lengths
     // turned into candidate offsets by a warp scan
     if (threadIdx.x < kDepRuns) {
       const int t = threadIdx.x, rw = row0 + (t >> 1), part = t & 1;
+      // x cells clo..clo+cnt-1 (mod C) of a (z, y) row: one or two contiguous runs
+      const int x0 = wrapi(s_clo[0], C), xend = x0 + s_cnt[0];
       int32_t pb = 0, len = 0;
-      if (rw < nrows && part < nparts) {
-        const int cz = wrapi(clo[2] + rw / cnt[1], C), cy = wrapi(clo[1] + rw % cnt[1], C);
+      if (rw < s_cnt[2] * s_cnt[1] && part <= (xend > C ? 1 : 0)) {
+        const int cz = wrapi(s_clo[2] + rw / s_cnt[1], C), cy = wrapi(s_clo[1] + rw % s_cnt[1], C);
         const int64_t row = ((int64_t)cz * C + cy) * C;
         const int ca = part == 0 ? x0 : 0, cb = part == 0 ? min(xend, C) : xend - C;
         pb = __ldg(a.begin + row + ca);
@@ -431,23 +438,23 @@ template <int T, int M>
 int launch_deposit_T(tpm_ctx* c, DepositArgs a) {
   a.ntile = ceil_div(c->N, T);
   const int blocks = a.ntile * a.ntile * a.ntile;
-  const size_t smem = sizeof(typename DepAcc<M>::T) * T * T * T + sizeof(int32_t) * kDepList;
+  const size_t smem = sizeof(typename DepAcc<M>::T) * T * T * T + sizeof(int32_t) * dep_list<M>;
   a.scale = 4.0 * M_PI * c->N;
   switch (c->opt.assign) {
     case TPM_ASSIGN_CIC:
       TPM_CUDA_TRY(cudaFuncSetAttribute(k_deposit<T, TPM_ASSIGN_CIC, M>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_deposit<T, TPM_ASSIGN_CIC, M><<<blocks, 256, smem, c->stream>>>(a);
+      k_deposit<T, TPM_ASSIGN_CIC, M><<<blocks, dep_threads<M>, smem, c->stream>>>(a);
       break;
     case TPM_ASSIGN_TSC:
       TPM_CUDA_TRY(cudaFuncSetAttribute(k_deposit<T, TPM_ASSIGN_TSC, M>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_deposit<T, TPM_ASSIGN_TSC, M><<<blocks, 256, smem, c->stream>>>(a);
+      k_deposit<T, TPM_ASSIGN_TSC, M><<<blocks, dep_threads<M>, smem, c->stream>>>(a);
       break;
     default:
       TPM_CUDA_TRY(cudaFuncSetAttribute(k_deposit<T, TPM_ASSIGN_CLOUD4, M>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_deposit<T, TPM_ASSIGN_CLOUD4, M><<<blocks, 256, smem, c->stream>>>(a);
+      k_deposit<T, TPM_ASSIGN_CLOUD4, M><<<blocks, dep_threads<M>, smem, c->stream>>>(a);
       break;
   }
   c->launches++;
