@@ -328,7 +328,7 @@ int tpm_batch_step(tpm_batch* b, int flags, int min_rung, double scale, double t
   if (!(flags & TPM_BATCH_GRAPH)) {
     const int64_t l0 = box_launches(b);
     const int rc = issue_step(b, flags, min_rung, scale, t0, first_call);
-    b->launches += box_launches(b) - l0 + 5;  // + queue (3), interp, kick
+    b->launches += box_launches(b) - l0 + 7;  // + queue (3), interp (2), kick (2)
     return rc;
   }
   const bool same = b->graph_ready && b->g_flags == flags && b->g_min_rung == min_rung && b->g_scale == scale &&

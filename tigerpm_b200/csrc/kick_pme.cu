@@ -112,6 +112,27 @@ __device__ __forceinline__ void q6(float x1, float* w, float* dw) {
   dw[5] = (7.f / 24.f) * y3 - (0.5f) * y4 + (5.f / 24.f) * y5;
 }
 
+// Packed weights of a z-run that starts s = 0..3 points into its first quad:
+// eight points in pairs, and the ninth (s = 3).
+__device__ __forceinline__ void shift_weights(const float (&w)[kNInterp], int s, f32x2 (&p)[4], float& last) {
+  float t[9];
+#pragma unroll
+  for (int m = 0; m < 9; m++) t[m] = m < kNInterp ? w[m] : 0.f;
+  if (s & 1) {
+#pragma unroll
+    for (int m = 8; m > 0; m--) t[m] = t[m - 1];
+    t[0] = 0.f;
+  }
+  if (s & 2) {
+#pragma unroll
+    for (int m = 8; m > 1; m--) t[m] = t[m - 2];
+    t[0] = t[1] = 0.f;
+  }
+#pragma unroll
+  for (int m = 0; m < 4; m++) p[m] = pack2(t[2 * m], t[2 * m + 1]);
+  last = t[8];
+}
+
 // Long-range force and potential at a sink: g = -sum dw.w.w phi N,
 // phi = sum w.w.w phi over the 6^3 points I-2..I+3 (periodic).  The cell
 // index and fraction come from the exact fixed-point product raw * N.
@@ -219,17 +240,89 @@ __device__ __forceinline__ void interp_long(const KickArgs& a, int4 q, float& lx
   lp = sp + pc;
 }
 
+// The same with the z weights in pairs (packed FMAs) and the loop over planes
+// unrolled, its weights in registers instead of local memory: at 128 registers
+// and 8 resident 64-thread blocks it replaces the form above at 85 registers
+// and 12 where the arguments are kernel parameters (2.98 against 3.07 ms at
+// 256^3 on a 768^3 mesh, 0.28 against 0.33 ms with a quarter of 128^3 sinks due,
+// 24 against 28 us at 32^3); with 12 blocks it spills (3.92 ms).  Runs that
+// wrap in z, and meshes whose rows are not whole quads, take the form above.
+__device__ __forceinline__ void interp_packed(const KickArgs& a, int4 q, float& lx, float& ly, float& lz,
+                                            float& lp) {
+  const int N = a.N;
+  float w[3][kNInterp], dw[3][kNInterp];
+  int base[3];
+  const uint32_t r[3] = {(uint32_t)q.x, (uint32_t)q.y, (uint32_t)q.z};
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const uint64_t t = (uint64_t)r[d] * (uint64_t)N;
+    base[d] = (int)(t >> 32) - 2;
+    q6((float)(uint32_t)t * 2.3283064365386963e-10f, w[d], dw[d]);
+  }
+  const int z0 = wrapi(base[2], N);
+  const int a4 = z0 & ~3;
+  if ((N & 3) != 0 || a4 + 12 > N) {
+    interp_long(a, q, lx, ly, lz, lp);
+    return;
+  }
+  int iy[kNInterp];
+#pragma unroll
+  for (int k = 0; k < kNInterp; k++) iy[k] = wrapi(base[1] + k, N) * N;
+  // sums over phi minus the stencil's centre value, as in interp_long
+  const float pc = __ldg(a.phi + (int64_t)wrapi(base[0] + 2, N) * N * N + iy[2] + z0 + 2);
+  float sx = 0.f, sy = 0.f, sz = 0.f, sp = 0.f;
+  const int s = z0 - a4;
+  f32x2 wz[4], dz[4];
+  float wl, dl;
+  shift_weights(w[2], s, wz, wl);
+  shift_weights(dw[2], s, dz, dl);
+  const f32x2 npc = pack2(-pc, -pc);
+#pragma unroll
+  for (int i = 0; i < kNInterp; i++) {
+    const int64_t plane = (int64_t)wrapi(base[0] + i, N) * N * N;
+    float px = 0.f, py = 0.f, pz = 0.f;
+#pragma unroll
+    for (int j = 0; j < kNInterp; j++) {
+      const float* row = a.phi + plane + iy[j] + a4;
+      const ulonglong2 f0 = __ldg(reinterpret_cast<const ulonglong2*>(row)),
+                       f1 = __ldg(reinterpret_cast<const ulonglong2*>(row) + 1);
+      const float f8 = s == 3 ? __ldg(row + 8) - pc : 0.f;
+      const f32x2 v[4] = {add2({f0.x}, npc), add2({f0.y}, npc), add2({f1.x}, npc), add2({f1.y}, npc)};
+      f32x2 rz2 = mul2(wz[0], v[0]), rd2 = mul2(dz[0], v[0]);
+#pragma unroll
+      for (int m = 1; m < 4; m++) {
+        rz2 = fma2(wz[m], v[m], rz2);
+        rd2 = fma2(dz[m], v[m], rd2);
+      }
+      const float2 zz = unpack2(rz2), dd = unpack2(rd2);
+      const float rz = fmaf(wl, f8, zz.x + zz.y), rdz = fmaf(dl, f8, dd.x + dd.y);
+      px = fmaf(w[1][j], rz, px);
+      py = fmaf(dw[1][j], rz, py);
+      pz = fmaf(w[1][j], rdz, pz);
+    }
+    sx = fmaf(dw[0][i], px, sx);
+    sy = fmaf(w[0][i], py, sy);
+    sz = fmaf(w[0][i], pz, sz);
+    sp = fmaf(w[0][i], px, sp);
+  }
+  lx = -sx * (float)N;
+  ly = -sy * (float)N;
+  lz = -sz * (float)N;
+  lp = sp + pc;
+}
+
 // Long-range part at every active sink of the kick box, stored in gx/gy/gz/pot
 // (unscaled); k_kick_pme adds the pair sums and applies GM.  Two kernels
 // compute it, one block per sink cell, chosen by the mesh points per sink.
 //
 // Direct form: one thread per sink, the 216 points read through L1.
-__device__ __forceinline__ void interp_cell_direct(const KickArgs& a, int64_t key, int min_rung) {
-  const int32_t pb = __ldg(a.begin + key), pe = __ldg(a.begin + key + 1);
+template <bool PACKED>
+__device__ __forceinline__ void interp_range(const KickArgs& a, int32_t pb, int32_t pe, int min_rung) {
   for (int32_t i = pb + (int32_t)threadIdx.x; i < pe; i += blockDim.x) {
     if (a.rung[i] < min_rung) continue;
     float lx, ly, lz, lp;
-    interp_long(a, __ldg(a.pos4 + i), lx, ly, lz, lp);
+    if (PACKED) interp_packed(a, __ldg(a.pos4 + i), lx, ly, lz, lp);
+    else interp_long(a, __ldg(a.pos4 + i), lx, ly, lz, lp);
     a.gx[i] = lx;
     a.gy[i] = ly;
     a.gz[i] = lz;
@@ -237,19 +330,19 @@ __device__ __forceinline__ void interp_cell_direct(const KickArgs& a, int64_t ke
   }
 }
 
-// 12 resident 64-thread blocks per SM (at most 85 registers): 2.55 ms against
-// 2.78 ms with the compiler's own choice at 256^3 on a 768^3 mesh
-#ifndef TPM_INTERP_MINB
-#define TPM_INTERP_MINB 12
-#endif
-__global__ void __launch_bounds__(64, TPM_INTERP_MINB) k_interp_direct(KickArgs a) {
+// cls: the work queue's cell classes; cells that it splits (more than
+// kSplitPasses passes of sinks) are left to k_interp_items.
+__device__ __forceinline__ bool split_cell(const int* cls, int64_t key) { return cls && (__ldg(cls + key) >> 6) > 1; }
+
+__global__ void __launch_bounds__(64, 8) k_interp_direct(KickArgs a, const int* __restrict__ cls) {
   int bid = blockIdx.x;
   const int i2 = bid % a.s2;
   bid /= a.s2;
   const int i1 = bid % a.s1;
   const int i0 = bid / a.s1;
-  const int C = a.C;
-  interp_cell_direct(a, ((int64_t)(a.b2 + i2) * C + (a.b1 + i1)) * C + (a.b0 + i0), a.min_rung);
+  const int64_t key = ((int64_t)(a.b2 + i2) * a.C + (a.b1 + i1)) * a.C + (a.b0 + i0);
+  if (split_cell(cls, key)) return;
+  interp_range<true>(a, __ldg(a.begin + key), __ldg(a.begin + key + 1), a.min_rung);
 }
 
 // The same interpolation from a shared-memory copy of the potential: one
@@ -303,7 +396,7 @@ __device__ __forceinline__ void interp_tile(const float* __restrict__ tile, int 
   lp = sp + pc;
 }
 
-__global__ void __launch_bounds__(128) k_interp_tile(KickArgs a, int maxw) {
+__global__ void __launch_bounds__(128) k_interp_tile(KickArgs a, int maxw, const int* __restrict__ cls) {
   extern __shared__ float tile[];
   int bid = blockIdx.x;
   const int i2 = bid % a.s2;
@@ -314,7 +407,7 @@ __global__ void __launch_bounds__(128) k_interp_tile(KickArgs a, int maxw) {
   const int cc[3] = {a.b0 + i0, a.b1 + i1, a.b2 + i2};
   const int64_t key = ((int64_t)cc[2] * C + cc[1]) * C + cc[0];
   const int32_t pb = __ldg(a.begin + key), pe = __ldg(a.begin + key + 1);
-  if (pb == pe) return;
+  if (pb == pe || split_cell(cls, key)) return;
   int o[3], W[3];
   bool fits = true;
 #pragma unroll
@@ -1065,26 +1158,42 @@ __global__ void k_item_scatter(const BoxCells* __restrict__ bc, int nbox, int to
   for (int p = 0; p < k; p++) items[at + p] = make_int4(b, key, p, p + 1);
 }
 
+// The sinks of the split cells, one queue item (a pass of npass sinks at most)
+// at a time; the items are alike, so blocks take them by stride.  A halo
+// cell of 30,000 sinks was one block's work before (3.1 -> 0.6 ms in a clustered
+// 128^3 box).
+template <bool SINGLE>
+__global__ void __launch_bounds__(64, 8)
+    k_interp_items(const KickArgs* __restrict__ boxes, KickArgs one, const int4* __restrict__ items,
+                   const int* __restrict__ nitems, int min_rung, int npass) {
+  const int n = __ldg(nitems + 1);
+  for (int it = blockIdx.x; it < n; it += gridDim.x) {
+    const int4 w = __ldg(items + it);  // (box, cell key, first pass, end pass)
+    const KickArgs a = SINGLE ? one : boxes[w.x];
+    const int32_t pb = __ldg(a.begin + w.y), pe = __ldg(a.begin + w.y + 1);
+    int np = 8;
+    while (np < npass && np < pe - pb) np <<= 1;
+    interp_range<true>(a, pb + w.z * np, (int32_t)min((int64_t)pe, (int64_t)pb + (int64_t)w.w * np), min_rung);
+  }
+}
+
 // Long-range interpolation of the batch: one block per global cell slot,
 // every box's cells in natural order, so that neighbouring cells' stencil
 // reads share the L1 and L2 as in the single-box k_interp_direct (in the
 // queue's cost order, items of different boxes interleave).
-__global__ void __launch_bounds__(64, TPM_INTERP_MINB)
-    k_interp_slots(const KickArgs* __restrict__ boxes, const BoxCells* __restrict__ bc, int nbox, int min_rung) {
+// 12 resident 64-thread blocks per SM (85 registers): with the arguments of its
+// box in registers the packed form is slower here (0.85 against 0.77 ms for 12
+// boxes of 32^3 to 96^3).
+__global__ void __launch_bounds__(64, 12)
+    k_interp_slots(const KickArgs* __restrict__ boxes, const BoxCells* __restrict__ bc, int nbox,
+                   const int* __restrict__ cls, int min_rung) {
   const int g = blockIdx.x;
+  const int c = __ldg(cls + g);
+  if (c < 0 || (c >> 6) > 1) return;  // empty, or in the items
   const int b = find_box(bc, nbox, g);
   const KickArgs a = boxes[b];  // the fields used, in registers
   const int key = g - __ldg(&bc[b].base);
-  const int32_t pb = __ldg(a.begin + key), pe = __ldg(a.begin + key + 1);
-  for (int32_t i = pb + (int32_t)threadIdx.x; i < pe; i += blockDim.x) {
-    if (a.rung[i] < min_rung) continue;
-    float lx, ly, lz, lp;
-    interp_long(a, __ldg(a.pos4 + i), lx, ly, lz, lp);
-    a.gx[i] = lx;
-    a.gy[i] = ly;
-    a.gz[i] = lz;
-    a.pot[i] = lp;
-  }
+  interp_range<false>(a, __ldg(a.begin + key), __ldg(a.begin + key + 1), min_rung);
 }
 
 // The batch's ordinary cells: one block per global cell slot (every box's
@@ -1187,8 +1296,9 @@ bool kick_shape_valid(const KickShape& k) {
          k.stage % 128 == 0 && pow2 && k.npass <= kPass && kick_smem(k) <= 200 * 1024;
 }
 
-int kick_queue_single(tpm_ctx* c, const KickArgs& a, const KickShape& k, int min_rung, double scale, double t0,
-                      int first_call, const int b[3], const int e[3]);
+int kick_queue_build(tpm_ctx* c, const KickArgs& a, const KickShape& k, const int b[3], const int e[3]);
+int kick_batch_launch(const BatchQueue& q, const KickShape& k, bool wrap, int min_rung, double scale, double t0,
+                      int first_call, cudaStream_t s, int* blocks_out, const KickArgs* single, bool split_only);
 
 int kick_pme(tpm_ctx* c, const int box[6], int min_rung, double scale, double t0, int first_call) {
   if (!c->sorted) return fail(TPM_ERR_STATE, "kick_pme needs chainmesh_create first");
@@ -1208,6 +1318,15 @@ int kick_pme(tpm_ctx* c, const int box[6], int min_rung, double scale, double t0
   const bool wrap = C == 3;
   auto kern = wrap ? k_kick_pme<true> : k_kick_pme<false>;
   TPM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const bool queue = ncell > 0 && !c->opt.kick_grid;
+  if (queue) {
+    const int rc = kick_queue_build(c, a, k, b, e);
+    if (rc) return rc;
+  }
+  const int* cls = queue ? c->kq.d_class : nullptr;
+  // Where the mean cell is one that the queue splits, the cells are alike and
+  // need no balancing: the interpolation takes them whole.
+  const bool apart = queue && mean_cell <= (double)kSplitPasses * k.npass;
   // Long-range interpolation.  A shared-memory tile of phi pays when a chain
   // cell's reach (its mesh span + 5 points per dim) is small against its
   // sinks (c2: 11.7^3 points for 184 sinks, 3.0 -> 2.1 ms); at 27 mesh cells
@@ -1219,26 +1338,29 @@ int kick_pme(tpm_ctx* c, const int box[6], int min_rung, double scale, double t0
   stage_begin(c, kStInterp);
   if (ncell > 0) {
     if (tile_bytes <= 48 * 1024 && span * span * span <= 16.0 * mean_cell) {
-      k_interp_tile<<<(unsigned)ncell, 128, tile_bytes, c->stream>>>(a, maxw);
+      k_interp_tile<<<(unsigned)ncell, 128, tile_bytes, c->stream>>>(a, maxw, apart ? cls : nullptr);
     } else {
-      k_interp_direct<<<(unsigned)ncell, 64, 0, c->stream>>>(a);
+      k_interp_direct<<<(unsigned)ncell, 64, 0, c->stream>>>(a, apart ? cls : nullptr);
     }
     c->launches++;
+    if (apart) {
+      k_interp_items<true><<<148 * 8, 64, 0, c->stream>>>(nullptr, a, c->kq.d_items, c->kq.d_nitems, min_rung, k.npass);
+      c->launches++;
+    }
     TPM_CUDA_TRY(cudaGetLastError());
   }
   stage_end(c, kStInterp);
   stage_begin(c, kStKick);
-  if (ncell > 0 && c->opt.kick_grid) {
-    kern<<<(unsigned)ncell, 32 * k.warps, smem, c->stream>>>(a, k.stage, k.npass, nullptr);
-    c->launches++;
-    TPM_CUDA_TRY(cudaGetLastError());
-  } else if (ncell > 0) {
+  if (ncell > 0) {
     // heavy cells' pass items through the persistent queue, every other cell
     // through the per-cell launch (faster for ordinary cells: 17.6 against
     // 18.6 ms at the 256^3 headline)
-    const int rc = kick_queue_single(c, a, k, min_rung, scale, t0, first_call, b, e);
-    if (rc) return rc;
-    kern<<<(unsigned)ncell, 32 * k.warps, smem, c->stream>>>(a, k.stage, k.npass, c->kq.d_class);
+    if (queue) {
+      const int rc = kick_batch_launch(c->kq, k, wrap, min_rung, scale, t0, first_call, c->stream, nullptr, &a, true);
+      if (rc) return rc;
+      c->launches++;
+    }
+    kern<<<(unsigned)ncell, 32 * k.warps, smem, c->stream>>>(a, k.stage, k.npass, cls);
     c->launches++;
     TPM_CUDA_TRY(cudaGetLastError());
   }
@@ -1296,10 +1418,12 @@ int kick_batch_queue(const BatchQueue& q, int npass, cudaStream_t s) {
 }
 
 int kick_batch_interp(const BatchQueue& q, int min_rung, int npass, cudaStream_t s) {
-  (void)npass;
   if (q.total_cells <= 0) return TPM_OK;
   k_interp_slots<<<(unsigned)q.total_cells, 64, 0, s>>>(static_cast<const KickArgs*>(q.d_args),
-                                                         static_cast<const BoxCells*>(q.d_cells), q.nbox, min_rung);
+                                                         static_cast<const BoxCells*>(q.d_cells), q.nbox, q.d_class,
+                                                         min_rung);
+  k_interp_items<false><<<148 * 8, 64, 0, s>>>(static_cast<const KickArgs*>(q.d_args), KickArgs{}, q.d_items, q.d_nitems,
+                                               min_rung, npass);
   TPM_CUDA_TRY(cudaGetLastError());
   return TPM_OK;
 }
@@ -1346,10 +1470,9 @@ int kick_batch_kick(const BatchQueue& q, const KickShape& k, bool wrap, int min_
   return TPM_OK;
 }
 
-// The single-box kick through the same persistent queue: heavy cells split
-// into pass items, so a strongly clustered box is spread over every SM.
-int kick_queue_single(tpm_ctx* c, const KickArgs& a, const KickShape& k, int min_rung, double scale, double t0,
-                      int first_call, const int b[3], const int e[3]) {
+// The single box's work queue: heavy cells split into pass items, so that a
+// strongly clustered box is spread over every SM.
+int kick_queue_build(tpm_ctx* c, const KickArgs& a, const KickShape& k, const int b[3], const int e[3]) {
   BatchQueue& q = c->kq;
   const int64_t ncell = (int64_t)c->C * c->C * c->C;
   if (!q.d_args) {
@@ -1385,10 +1508,8 @@ int kick_queue_single(tpm_ctx* c, const KickArgs& a, const KickShape& k, int min
   }
   TPM_CUDA_TRY(cudaMemcpyAsync(q.d_args, ha, sizeof(KickArgs), cudaMemcpyHostToDevice, c->stream));
   TPM_CUDA_TRY(cudaMemcpyAsync(q.d_cells, hb, sizeof(BoxCells), cudaMemcpyHostToDevice, c->stream));
-  int rc = kick_batch_queue(q, k.npass, c->stream);
-  if (rc == TPM_OK) rc = kick_batch_launch(q, k, c->C == 3, min_rung, scale, t0, first_call, c->stream, nullptr, &a, true);
-  c->launches += 4;
-  return rc;
+  c->launches += 3;
+  return kick_batch_queue(q, k.npass, c->stream);
 }
 
 }  // namespace tpm
