@@ -484,9 +484,9 @@ __device__ __forceinline__ void soften(const PairK& k, float r2, float& rinv3, f
 // scalar one 1.5) and the MUFU (8 cycles a result and warp, 3 results a pair)
 // about equally: in isolation 16 sources x 8 sinks take a warp 89 instructions
 // and 137 cycles of an SM quarter, 130 and 157 as scalars.  Kick at 256^3:
-// 14.30 -> 13.43 ms on the 768^3 mesh, 41.6 -> 33.1 ms on the literal mesh;
-// 88.0 -> 67 ms for the reference's options at 90^3 (packed pairs, groups by
-// halves and the 64-source cull step together).
+// 14.30 -> 13.4 ms on the 768^3 mesh, 41.6 -> 32.9 ms on the literal mesh;
+// 88.0 -> 60 ms for the reference's options at 90^3 (packed pairs, groups by
+// halves, the 64-source cull step and no cull without a cutoff together).
 //
 // WRAP folds the offset to the minimum image, as the reference's int32
 // difference does; it is needed only when chain_dim = 3, where the 27 cells
@@ -506,7 +506,8 @@ __device__ __forceinline__ void soften(const PairK& k, float r2, float& rinv3, f
 // kernel (r <= h, the sink itself included) is entered on one warp vote.
 // count: sources from this lane's first one on that exist (WRAP only; without
 // it the caller pads with far sources).
-template <bool WRAP, int NP>
+// CUT: pairs beyond the cutoff are taken out (without a cutoff there are none).
+template <bool WRAP, bool CUT, int NP>
 __device__ __forceinline__ void pairs(const PairK& k, const f32x2 (&ns)[3], const f32x2 (&s)[3][NP], f32x2 (&sum)[4],
                                       int count) {
   f32x2 d[3][NP], f[NP], q[NP];
@@ -533,7 +534,8 @@ __device__ __forceinline__ void pairs(const PairK& k, const f32x2 (&ns)[3], cons
     // vanish and the pair adds exactly 0, without a mask on the results.
     // Pairs at r <= h (r = 0 too) take the softened kernel, which replaces
     // every term formed here.
-    const float a = r2[2 * i] < k.rcut2 ? r2[2 * i] : 1e30f, b = r2[2 * i + 1] < k.rcut2 ? r2[2 * i + 1] : 1e30f;
+    const float a = !CUT || r2[2 * i] < k.rcut2 ? r2[2 * i] : 1e30f;
+    const float b = !CUT || r2[2 * i + 1] < k.rcut2 ? r2[2 * i + 1] : 1e30f;
     const f32x2 rinv = pack2(rsqrt_approx(a), rsqrt_approx(b));
     const float2 w = unpack2(fma2(pack2(a, b), rinv, pack2(kInvP, kInvP)));
     const f32x2 t = pack2(rcp_approx(w.x), rcp_approx(w.y));
@@ -608,7 +610,12 @@ constexpr float kFar = 1e18f;     // offset of a padding source: beyond any cuto
 // the power of two >= the cell's count, at most npass); every thread of the
 // block calls it with the same arguments.  A pass streams the whole 27-cell
 // neighbourhood, so the passes of one cell are independent work items.
-template <bool WRAP>
+//
+// CULL: sources are culled against the groups' boxes.  Without a cutoff, or
+// under the minimum image (the cull works on unwrapped offsets), every source
+// is kept and the pairs come straight from the stage (the reference's options
+// at 90^3: 71 ms through the cull and its buffer, 60 ms without).
+template <bool WRAP, bool CULL>
 __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int cz, float4* smem4, int stage,
                                           int npass, int pass_lo = 0, int pass_hi = 0x7fffffff) {
   const int T = blockDim.x, W = T >> 5;
@@ -631,8 +638,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
   // offsets, cutoff and softening length in units of 2 r_s / sqrt(log2 e)
   // (see pairs())
   const PairK pk{a.rcut2, a.h2, a.wlen};
-  // culling works on unwrapped offsets; without it every source is kept
-  const float ck = WRAP ? 0.f : a.cull_k, cm = WRAP ? 0.f : a.cull_m;
+  const float ck = a.cull_k, cm = a.cull_m;
   uint32_t* org = mask + kPass / 32;  // the cell's centre, not in registers through the pair loop
   if (tid < 3) org[tid] = (uint32_t)((((uint64_t)(2 * (tid == 0 ? cx : tid == 1 ? cy : cz) + 1)) << 31) / (uint64_t)C);
   if (warp == 0) {
@@ -708,7 +714,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
     // being its range's start plus the number of smaller keys in the range
     // (keys are unique).  Groups of 8 keep 2.2 candidates per pair inside the
     // cutoff at 64 sinks per cell (1.8 at 184), Morton order 2.5 (2.1).
-    if (!WRAP && ck != 0.f) {
+    if (CULL) {
       const int pad = (ngroups * kGroup) - nact;  // the last group's absent sinks sort last
       if (tid < pad) from[nact + tid] = from[npass + nact + tid] = from[2 * npass + nact + tid] = 0xffffffffu;
       __syncthreads();
@@ -782,7 +788,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
         float byl = mysink ? sp.y : INFINITY, byh = mysink ? sp.y : -INFINITY;
         float bzl = mysink ? sp.z : INFINITY, bzh = mysink ? sp.z : -INFINITY;
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1) {
+        for (int o = CULL ? 4 : 0; o > 0; o >>= 1) {
           bxl = fminf(bxl, __shfl_xor_sync(0xffffffffu, bxl, o));
           bxh = fmaxf(bxh, __shfl_xor_sync(0xffffffffu, bxh, o));
           byl = fminf(byl, __shfl_xor_sync(0xffffffffu, byl, o));
@@ -795,8 +801,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
         // distance of a cutoff or more is no candidate whatever the other
         // axes are).  The half-extent is widened by cull_m to cover the
         // rounding of c, h and s - c, so the cull never drops a source the
-        // exact pair test keeps.  Without a cutoff all scales are 0 and every
-        // source is kept.
+        // exact pair test keeps.
         const f32x2 k2 = pack2(ck, ck);
         const float nx = -0.5f * (bxl + bxh) * ck, ny = -0.5f * (byl + byh) * ck, nz = -0.5f * (bzl + bzh) * ck;
         const f32x2 ncx = pack2(nx, nx), ncy = pack2(ny, ny), ncz = pack2(nz, nz);
@@ -806,6 +811,19 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
         f32x2 sum[4];
 #pragma unroll
         for (int c = 0; c < 4; c++) sum[c] = pack2(0.f, 0.f);
+        if constexpr (!CULL) {
+          // the chunk is padded to whole steps of 64 with far sources; under
+          // the minimum image the count leaves them out
+#pragma unroll 1
+          for (int t = 0; t < len; t += 16) {
+            const float* p = src + t + 4 * ph;
+            const ulonglong2 ux = *reinterpret_cast<const ulonglong2*>(p);
+            const ulonglong2 uy = *reinterpret_cast<const ulonglong2*>(p + stage);
+            const ulonglong2 uz = *reinterpret_cast<const ulonglong2*>(p + 2 * stage);
+            const f32x2 u[3][2] = {{{ux.x}, {ux.y}}, {{uy.x}, {uy.y}}, {{uz.x}, {uz.y}}};
+            pairs<WRAP, WRAP, 2>(pk, ns, u, sum, len - t - 4 * ph);
+          }
+        } else {
         int cnt = 0;   // buffered sources
         int head = 0;  // ring position of the first of them: 0 or kFlush
         // Every lane tests two staged sources; kept ones are appended to the
@@ -821,11 +839,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
           const f32x2 ey = pack2(__saturatef(fabsf(dy.x) - hy), __saturatef(fabsf(dy.y) - hy));
           const f32x2 ez = pack2(__saturatef(fabsf(dz.x) - hz), __saturatef(fabsf(dz.y) - hz));
           const float2 d2 = unpack2(fma2(ex, ex, fma2(ey, ey, mul2(ez, ez))));
-          bool k0 = d2.x < 1.0f, k1 = d2.y < 1.0f;
-          if (WRAP) {  // no far padding under the minimum image
-            k0 = k0 && j < len;
-            k1 = k1 && j + 1 < len;
-          }
+          const bool k0 = d2.x < 1.0f, k1 = d2.y < 1.0f;
           const unsigned b0 = __ballot_sync(0xffffffffu, k0), b1 = __ballot_sync(0xffffffffu, k1);
           const int at = head + cnt + __popc(b0 & lt) + __popc(b1 & lt);
           const float2 x = unpack2(sx), y = unpack2(sy), z = unpack2(sz);
@@ -853,18 +867,17 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
               const ulonglong2 uy = *reinterpret_cast<const ulonglong2*>(p + kBuf);
               const ulonglong2 uz = *reinterpret_cast<const ulonglong2*>(p + 2 * kBuf);
               const f32x2 u[3][2] = {{{ux.x}, {ux.y}}, {{uy.x}, {uy.y}}, {{uz.x}, {uz.y}}};
-              pairs<WRAP, 2>(pk, ns, u, sum, 4);
+              pairs<WRAP, true, 2>(pk, ns, u, sum, 4);
             }
             cnt -= kFlush;
             head ^= kFlush;
             __syncwarp();
           }
         }
-        // the rest, 8 sources a step: padded with far ones (under the
-        // minimum image with zeros that count excludes)
+        // the rest, 8 sources a step: padded with far ones
         if (lane < ((8 - (cnt & 7)) & 7)) {
           float* p = buf + ((head + cnt + lane) & (kBuf - 1));
-          p[0] = p[kBuf] = p[2 * kBuf] = WRAP ? 0.f : kFar;
+          p[0] = p[kBuf] = p[2 * kBuf] = kFar;
         }
         __syncwarp();
         for (int t = 0; t < cnt; t += 8) {
@@ -872,7 +885,8 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
           const f32x2 u[3][1] = {{*reinterpret_cast<const f32x2*>(p)},
                                  {*reinterpret_cast<const f32x2*>(p + kBuf)},
                                  {*reinterpret_cast<const f32x2*>(p + 2 * kBuf)}};
-          pairs<WRAP, 1>(pk, ns, u, sum, cnt - t - 2 * ph);
+          pairs<WRAP, true, 1>(pk, ns, u, sum, cnt - t - 2 * ph);
+        }
         }
         float px, py, pz, pp;
         {
@@ -957,7 +971,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
 // One block per sink cell.  split (optional): the queue's per-cell class
 // words; cells split into pass items (more than kSplitPasses passes) are left
 // to the persistent launch over those items.
-template <bool WRAP>
+template <bool WRAP, bool CULL>
 __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
     k_kick_pme(KickArgs a, int stage, int npass, const int* __restrict__ split) {
   extern __shared__ float4 smem4[];
@@ -968,7 +982,7 @@ __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
   const int i0 = bid / a.s1;
   const int cx = a.b0 + i0, cy = a.b1 + i1, cz = a.b2 + i2;
   if (split && (__ldg(split + ((int64_t)cz * a.C + cy) * a.C + cx) >> 6) > 1) return;
-  kick_cell<WRAP>(a, cx, cy, cz, smem4, stage, npass);
+  kick_cell<WRAP, CULL>(a, cx, cy, cz, smem4, stage, npass);
 }
 
 // ------------------------------------------------------------ batched kick
@@ -996,7 +1010,7 @@ __device__ __forceinline__ KickArgs box_args(const KickArgs* __restrict__ boxes,
 // SINGLE: one box whose arguments come as the kernel parameter `one` (the
 // constant bank, like the per-cell launch); else per-box arguments from
 // `boxes`, kept in shared memory.
-template <bool WRAP, bool SINGLE>
+template <bool WRAP, bool CULL, bool SINGLE>
 __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
     k_kick_batch(const KickArgs* __restrict__ boxes, KickArgs one, const int4* __restrict__ items,
                  const int* __restrict__ nitems, int* __restrict__ counter, StepScalars st, int stage, int npass) {
@@ -1021,7 +1035,7 @@ __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
     if (w.x >= 0) {  // uniform: every thread read the same item
       if (SINGLE) {
         const int C = one.C;
-        kick_cell<WRAP>(one, w.y % C, (w.y / C) % C, w.y / (C * C), smem4, stage, npass, w.z, w.w);
+        kick_cell<WRAP, CULL>(one, w.y % C, (w.y / C) % C, w.y / (C * C), smem4, stage, npass, w.z, w.w);
       } else {
         if (w.x != cur_box) {
           if (threadIdx.x == 0) s_args = box_args(boxes, w.x, st);
@@ -1029,7 +1043,7 @@ __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
           __syncthreads();
         }
         const int C = s_args.C;
-        kick_cell<WRAP>(s_args, w.y % C, (w.y / C) % C, w.y / (C * C), smem4, stage, npass, w.z, w.w);
+        kick_cell<WRAP, CULL>(s_args, w.y % C, (w.y / C) % C, w.y / (C * C), smem4, stage, npass, w.z, w.w);
       }
     }
     __syncthreads();
@@ -1212,7 +1226,7 @@ __global__ void __launch_bounds__(kKickThreads, TPM_KICK_MINB)
   __syncthreads();
   const int key = g - __ldg(&bc[b].base);
   const int C = s_args.C;
-  kick_cell<WRAP>(s_args, key % C, (key / C) % C, key / (C * C), smem4, stage, npass);
+  kick_cell<WRAP, !WRAP>(s_args, key % C, (key / C) % C, key / (C * C), smem4, stage, npass);
 }
 
 }  // namespace
@@ -1316,7 +1330,7 @@ int kick_pme(tpm_ctx* c, const int box[6], int min_rung, double scale, double t0
   const KickShape k = kick_default_shape(mean_cell);
   const size_t smem = kick_smem(k);
   const bool wrap = C == 3;
-  auto kern = wrap ? k_kick_pme<true> : k_kick_pme<false>;
+  auto kern = wrap ? k_kick_pme<true, false> : c->rcut_box > 0 ? k_kick_pme<false, true> : k_kick_pme<false, false>;
   TPM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool queue = ncell > 0 && !c->opt.kick_grid;
   if (queue) {
@@ -1433,8 +1447,10 @@ int kick_batch_launch(const BatchQueue& q, const KickShape& k, bool wrap, int mi
   if (!kick_shape_valid(k)) return fail(TPM_ERR_INVALID, "invalid kick shape");
   if (q.total_cells <= 0) return TPM_OK;
   const size_t smem = kick_smem(k);
-  auto kern = single ? (wrap ? k_kick_batch<true, true> : k_kick_batch<false, true>)
-                     : (wrap ? k_kick_batch<true, false> : k_kick_batch<false, false>);
+  // a batch's boxes may differ in their cutoffs: those without one keep every source
+  auto kern = single ? (wrap ? k_kick_batch<true, false, true>
+                             : single->cull_k > 0.f ? k_kick_batch<false, true, true> : k_kick_batch<false, false, true>)
+                     : (wrap ? k_kick_batch<true, false, false> : k_kick_batch<false, true, false>);
   TPM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0, dev = 0, sms = 0;
   TPM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * k.warps, smem));
