@@ -14,7 +14,8 @@
 //   queue   every non-empty (box, chain cell) becomes a work item, bucketed
 //           by the binary order of magnitude of its cost (sinks x
 //           neighbourhood sources), heaviest bucket first
-//   interp  long-range interpolation of every item, one launch
+//   interp  long-range interpolation: one launch over the cells, one over the
+//           pass items of split cells
 //   kick    ONE persistent launch: resident blocks take items from a global
 //           counter until the queue is empty (PP sum + rung kick)
 //

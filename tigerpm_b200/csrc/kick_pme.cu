@@ -12,7 +12,8 @@
 //  * No host staging: particles are already in chain-cell order on the device
 //    and the 27 neighbours of a cell are 9 contiguous (z, y) rows of three x
 //    cells (two runs where x wraps), read straight from cell offsets.
-//  * The interpolation is its own kernel (one block per chain cell), run just
+//  * The interpolation is its own kernel (one block per chain cell; cells that
+//    the work queue splits, one block per pass of sinks), run just
 //    before the pair kernel; its results stay in L2 for the kick.
 //  * Pair kernel, one block per sink cell.  Sources are staged in shared
 //    memory as float offsets from the sink cell centre: the int32
@@ -586,10 +587,11 @@ __device__ __forceinline__ unsigned order_key(int x, uint32_t o, int C, int slot
 }
 
 // Work decomposition.  A block owns one sink cell.  Its active sinks (up to
-// kPass per pass) are cut into groups of kGroup = 8 (compact in space).  Warps take groups round-robin.  For each group a warp streams the
-// staged neighbourhood 64 at a time (two per lane), keeps the sources within
-// rcut of the group's bounding box (ballot + popc) and copies them into its
-// ring buffer; lanes are (sink t = lane % 8) x (phase = lane / 8), so one
+// kPass per pass) are cut into groups of kGroup = 8 (compact in space).  Warps
+// take groups round-robin.  For each group a warp streams the staged
+// neighbourhood 64 at a time (two per lane), keeps the sources within rcut of
+// the group's bounding box (ballot + popc) and copies them into its ring
+// buffer; lanes are (sink t = lane % 8) x (phase = lane / 8), so one
 // step evaluates 8 sinks against 16 consecutive buffered sources, 4 per lane,
 // and a fixed two-step shuffle reduction folds the 4 phases.  Sources are
 // staged and buffered as separate x, y and z arrays, so that a 16-byte load
@@ -597,7 +599,9 @@ __device__ __forceinline__ unsigned order_key(int x, uint32_t o, int C, int slot
 // compensation across chunks.
 //
 // Shared memory (dynamic): src[3][stage] float | buf[W][3][kBuf] float |
-// spos[kPass] float4 | acc[kPass][8] float | skey[kPass] | runb/runp.
+// spos[kPass] float4 | acc[kPass][8] float (before the sums: two sets of the
+// grouping's three key arrays) | sidx[kPass] byte | run table | active masks |
+// cell centre and pass bounds.
 constexpr int kPass = 256;
 constexpr int kGroup = 8;
 constexpr int kFlush = 64;        // buffered sources evaluated at a time
