@@ -332,9 +332,15 @@ int tpm_pme_steps_host(tpm_ctx* ctx, int64_t nsteps, int64_t n, const tpm_host_p
                        const tpm_host_particles* out, int min_rung, double scale, double t0,
                        int first_call);
 /* Synchronises and reports (then clears) device error flags raised since the
- * last check: TPM_ERR_RUNG for a clamped rung, TPM_ERR_INVALID for a drift
- * step beyond 2^31 box lengths. */
+ * last check: TPM_ERR_TIMEOUT for a bounded device wait that gave up,
+ * TPM_ERR_RUNG for a clamped rung, TPM_ERR_INVALID for a drift step beyond
+ * 2^31 box lengths. */
 int tpm_check_errors(tpm_ctx* ctx);
+/* Polls of one bounded device wait (the sort's look-back) before it gives up;
+ * the default is 2^22, about a second.  At 0 every such wait gives up at once,
+ * which shows a program what a timeout looks like: the particles keep an order
+ * that is not the chain mesh's, and the next check reports TPM_ERR_TIMEOUT. */
+int tpm_set_wait_limit(tpm_ctx* ctx, int64_t polls);
 
 /* ------------------------------------------------------- integration
  *

@@ -1,0 +1,42 @@
+"""A look-back wait of the sort that gives up: the sort ends, every particle is
+still there exactly once, the timeout is reported, and the context sorts
+correctly afterwards.  The limit is set to zero polls, so that waits run out at
+once on sets that need them (more than one scan tile of 4,096)."""
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import oracle_particles, with_random_motion
+from tigerpm_b200 import _lib
+from tigerpm_b200 import workloads as W
+from tigerpm_b200.api import GRAVITY_LONG_PME, TigerPM, TPMError, make_options
+
+pytestmark = pytest.mark.gpu
+
+
+def rows(arrays):
+    x, y, z, vx, vy, vz, r = arrays
+    a = np.stack([x, y, z, vx.view(np.uint32), vy.view(np.uint32), vz.view(np.uint32), r.astype(np.uint32)])
+    return a[:, np.lexsort(a)]
+
+
+@pytest.mark.parametrize("n,C", [(9000, 3), (50000, 16), (300000, 17), (300000, 64), (4300000, 20)])
+def test_sort_that_gave_up_keeps_every_particle(n, C):
+    ps = with_random_motion(W.uniform(n, n), n)
+    with TigerPM(make_options(max(2, round(n ** (1 / 3))), 16, chain=C), n) as t:
+        t.set_wait_limit(0)
+        t.set_particles(ps)
+        t.chainmesh_create()
+        assert np.array_equal(rows(t.get_particles()), rows(ps.arrays()))
+        with pytest.raises(TPMError) as e:
+            t.check_errors()
+        assert e.value.status == _lib.TPM_ERR_TIMEOUT
+        t.check_errors()  # reported once
+        t.set_wait_limit(1 << 22)
+        t.set_particles(ps)
+        t.chainmesh_create()
+        t.check_errors()
+        x, y, z, *_ = t.get_particles()
+        p = oracle_particles(O, ps)
+        O.chainmesh_sort(C, p)
+        assert np.array_equal(x, p.x) and np.array_equal(y, p.y) and np.array_equal(z, p.z)

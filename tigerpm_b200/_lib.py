@@ -155,6 +155,7 @@ SIGNATURES = [
     ("tpm_pme_step", _I, [_P, _I, _D, _D, _I]),
     ("tpm_pme_steps_host", _I, [_P, _I64, _I64, _P, _P, _I, _D, _D, _I]),
     ("tpm_check_errors", _I, [_P]),
+    ("tpm_set_wait_limit", _I, [_P, _I64]),
     ("tpm_batch_create", _I, [_I, C.POINTER(Options), C.POINTER(_I64), C.POINTER(_P)]),
     ("tpm_batch_destroy", _I, [_P]),
     ("tpm_batch_size", _I, [_P, C.POINTER(_I), C.POINTER(_I64)]),

@@ -393,6 +393,10 @@ class TigerPM:
     def check_errors(self) -> None:
         check(self.lib.tpm_check_errors(self.h), "check_errors")
 
+    def set_wait_limit(self, polls: int) -> None:
+        """Polls of a bounded device wait before it gives up (0: at once)."""
+        check(self.lib.tpm_set_wait_limit(self.h, int(polls)), "set_wait_limit")
+
     def count_pairs(self, min_rung: int = 0):
         a = C.c_int64()
         b = C.c_int64()

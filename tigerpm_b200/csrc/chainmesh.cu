@@ -279,8 +279,11 @@ __device__ __forceinline__ unsigned long long pack_status(unsigned stamp, unsign
 // matter only to the node that runs into it (chained scan with decoupled
 // look-back; tiles are taken in launch order through an atomic counter, so
 // every predecessor a tile waits on is already running).  The look-back is
-// done by one warp, 32 predecessor tiles at a time; its spin is bounded: on
-// expiry the tile records kErrTimeout and uses what it has summed.
+// done by one warp, 32 predecessor tiles at a time; its polls are bounded: at
+// the limit the tile records kErrTimeout, sets *gave_up and uses what it has
+// summed.  Counts and slots are then wrong (though in range), so no level
+// swaps from there on and the units keep their order: the result is still a
+// permutation of the particles.
 //
 // Bound by latency and issue (36 us per level of 7.65e6 particles, 31 MB read):
 // 4 bytes of key read per position, 4 written per misplaced one.  Nodes come
@@ -289,7 +292,8 @@ __device__ __forceinline__ unsigned long long pack_status(unsigned stamp, unsign
 // prefix array, a slot pass and a swap pass they took 145 us.
 __global__ void __launch_bounds__(kScanThreads, 4)
     k_level_scan(LevelArgs a, unsigned stamp, int* __restrict__ counter, unsigned long long* __restrict__ status,
-                 int32_t* __restrict__ slot, int32_t* __restrict__ misplaced, int4* __restrict__ heads, int* __restrict__ err) {
+                 int32_t* __restrict__ slot, int32_t* __restrict__ misplaced, int4* __restrict__ heads, long long polls,
+                 int* __restrict__ gave_up, int* __restrict__ err) {
   __shared__ int warp_tot[32];
   __shared__ int total;
   __shared__ unsigned tile_s;
@@ -351,6 +355,13 @@ __global__ void __launch_bounds__(kScanThreads, 4)
         int top = (int)tile - 1;
         long long spins = 0;
         while (true) {
+          if (spins++ >= polls) {
+            if (lane == 0) {
+              atomicExch(gave_up, 1);
+              atomicOr(err, kErrTimeout);
+            }
+            break;
+          }
           const int j = top - lane;
           unsigned long long f = kFlagIncl;  // before tile 0: a complete zero
           int v = 0;
@@ -359,13 +370,8 @@ __global__ void __launch_bounds__(kScanThreads, 4)
             f = (unsigned)(w >> 34) == stamp ? (w >> 32) & 3ull : 0ull;
             v = (int)(unsigned)(w & 0xffffffffull);
           }
-          if (__any_sync(0xffffffffu, f == 0)) {
-            if (++spins > (1ll << 22)) {
-              if (lane == 0) atomicOr(err, kErrTimeout);
-              break;
-            }
-            continue;
-          }
+          if (__any_sync(0xffffffffu, f == 0)) continue;
+          spins = 0;
           const unsigned incl = __ballot_sync(0xffffffffu, f == kFlagIncl);
           const int nearest = incl ? __ffs(incl) - 1 : 32;
           int sum = lane <= nearest ? v : 0;
@@ -419,8 +425,9 @@ __global__ void __launch_bounds__(kScanThreads, 4)
 // lookup.
 __global__ void __launch_bounds__(256) k_level_swap(LevelArgs a, const int32_t* __restrict__ misplaced,
                                                     const int32_t* __restrict__ slot, const int4* __restrict__ heads,
-                                                    uint32_t* __restrict__ key, int32_t* __restrict__ idx) {
-  if (a.big_only && *a.nbig == 0) return;
+                                                    const int* __restrict__ gave_up, uint32_t* __restrict__ key,
+                                                    int32_t* __restrict__ idx) {
+  if ((a.big_only && *a.nbig == 0) || *gave_up) return;
   const unsigned n = (unsigned)a.n;
   for (unsigned blk = blockIdx.x; blk < (n + kSwapBlock - 1) / kSwapBlock; blk += gridDim.x) {
     const int4 h = __ldg(heads + blk);
@@ -437,9 +444,8 @@ __global__ void __launch_bounds__(256) k_level_swap(LevelArgs a, const int32_t* 
       if (!nd.live || p >= (unsigned)nd.pm) continue;
       if (wrong < 0) wrong = __ldg(misplaced + nd.b);
       const int32_t i = (int32_t)(p - nd.b);
-      if (i >= wrong || nd.pm + i >= nd.e) continue;
+      if (i >= wrong) continue;
       const int32_t u = __ldg(slot + p), v = __ldg(slot + nd.pm + i);
-      if ((unsigned)u >= n || (unsigned)v >= n) continue;  // after a look-back gave up
       const uint32_t ku = key[u], kv = key[v];
       const int32_t iu = idx[u], iv = idx[v];
       key[u] = kv;
@@ -467,6 +473,7 @@ struct UnitArgs {
   int32_t* __restrict__ out;
   int* __restrict__ nbig;
   int* __restrict__ njump;
+  const int* __restrict__ gave_up;
 };
 
 __device__ __forceinline__ void unit_cells(const UnitArgs& a, int u, int64_t& c0, int64_t& c1) {
@@ -516,7 +523,10 @@ __global__ void __launch_bounds__(kFinishThreads, 2) k_finish(UnitArgs a) {
   const int n = __ldg(a.begin + c1) - b0;
   const int cells = (int)(c1 - c0);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (n > kUnit) {  // sorted by the level kernels
+  // Left as it is: a unit that the level kernels sort, and every unit once a
+  // look-back gave up (its elements may then belong to any cell, and the tables
+  // below are read by the element's cell).
+  if (n > kUnit || *a.gave_up) {
     for (int i = tid; i < n; i += kFinishThreads) a.out[b0 + i] = a.idx[b0 + i];
     return;
   }
@@ -807,14 +817,14 @@ int partition(tpm_ctx* c, int64_t n) {
   cudaStream_t s = c->stream;
   const int nb = ceil_div(n, kScanTile), depth = c->max_depth1d;
   const FinishStart f = finish_start(c, n);
-  // look-back words, then a tile counter per level and the count of big units
+  // look-back words, then a tile counter per level and the sort's other counters
   unsigned long long* status = c->scan_status;
   int* counters = reinterpret_cast<int*>(status + nb);
   TPM_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * nb + sizeof(int) * kSortCounters, s));
   int* nbig = counters + kSortBig;
   const UnitLevel ul = f.udim < 0 ? UnitLevel{} : c->unit_levels[f.ulevel];
   UnitArgs u{C, f.udim, f.ulevel, ul.count, c->unit_cuts + ul.at, c->cell_begin, c->tree, c->depth1d, depth, c->key,
-             c->idx, c->prefix, nbig, counters + kSortJumps};
+             c->idx, c->prefix, nbig, counters + kSortJumps, counters + kSortGaveUp};
   const int64_t units = f.udim < 0 ? 0 : (f.udim == 2 ? 1 : f.udim == 1 ? (int64_t)C : (int64_t)C * C) * u.cuts_n;
   if (n > kUnit && units > 0) {
     k_big_units<<<ceil_div(units, 256), 256, 0, s>>>(u, (int)units);
@@ -832,8 +842,8 @@ int partition(tpm_ctx* c, int64_t n) {
       LevelArgs a{n, C, dim, level, f.udim, f.ulevel, below ? 1 : 0, nbig, c->cellof, c->key, c->cell_begin, c->tree,
                   c->depth1d};
       k_level_scan<<<scan_blocks, kScanThreads, 0, s>>>(a, (unsigned)(l + 1), counters + l, status, c->slot, c->prefix,
-                                                         heads, c->d_err);
-      k_level_swap<<<swap_blocks, 256, 0, s>>>(a, c->prefix, c->slot, heads, c->key, c->idx);
+                                                         heads, c->wait_polls, counters + kSortGaveUp, c->d_err);
+      k_level_swap<<<swap_blocks, 256, 0, s>>>(a, c->prefix, c->slot, heads, counters + kSortGaveUp, c->key, c->idx);
       c->launches += 2;
     }
   if (units > 0) {

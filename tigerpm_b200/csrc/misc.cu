@@ -123,6 +123,12 @@ int tpm_check_errors(tpm_ctx* c) {
   return TPM_OK;
 }
 
+int tpm_set_wait_limit(tpm_ctx* c, int64_t polls) {
+  if (!c || polls < 0) return fail(TPM_ERR_INVALID, "null context or negative limit");
+  c->wait_polls = polls;
+  return TPM_OK;
+}
+
 int tpm_count_pairs(tpm_ctx* c, int min_rung, int64_t* candidates, int64_t* inside) {
   if (!c || !candidates || !inside) return fail(TPM_ERR_INVALID, "null argument");
   if (!c->sorted) return fail(TPM_ERR_STATE, "count_pairs needs chainmesh_create first");
