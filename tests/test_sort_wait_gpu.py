@@ -1,6 +1,6 @@
 """A look-back wait of the sort that gives up: the sort ends, every particle is
 still there exactly once, the timeout is reported, and the context sorts
-correctly afterwards.  The limit is set to zero polls, so that waits run out at
+correctly afterwards; and every call that reports device errors reports it.  The limit is set to zero polls, so that waits run out at
 once on sets that need them (more than one scan tile of 4,096)."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ import oracle as O
 from helpers import oracle_particles, with_random_motion
 from tigerpm_b200 import _lib
 from tigerpm_b200 import workloads as W
-from tigerpm_b200.api import GRAVITY_LONG_PME, TigerPM, TPMError, make_options
+from tigerpm_b200.api import GRAVITY_LONG_PME, Server, TigerPM, TPMError, make_options
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,29 @@ def test_sort_that_gave_up_keeps_every_particle(n, C):
         p = oracle_particles(O, ps)
         O.chainmesh_sort(C, p)
         assert np.array_equal(x, p.x) and np.array_equal(y, p.y) and np.array_equal(z, p.z)
+
+
+def test_every_reporting_call_reports_the_timeout():
+    ps = with_random_motion(W.uniform(20000, 2), 2)
+    opts = make_options(27, 32, chain=6, rs_cells=1.0, rcut_over_rs=4.5)
+    with TigerPM(opts, ps.n) as t:
+        t.set_wait_limit(0)
+
+        def step(last):
+            t.set_particles(ps)
+            t.chainmesh_create()
+            t.gravity_long_compute(GRAVITY_LONG_PME)
+            with pytest.raises(TPMError) as e:
+                last()
+            assert e.value.status == _lib.TPM_ERR_TIMEOUT
+            t.check_errors()
+
+        step(lambda: t.kick_pme_begin(0, 1.0, 0.01, False))
+        step(lambda: t.drift(0.01))
+        step(lambda: t.integrate(0.01))
+    with Server(max_slots=1) as s:
+        b = s.add_box(opts, ps)
+        s.box(b).set_wait_limit(0)
+        with pytest.raises(TPMError) as e:
+            s.wait(s.submit(b, 0.01, t0=0.01, first_call=False))
+        assert e.value.status == _lib.TPM_ERR_TIMEOUT

@@ -95,8 +95,7 @@ int check_err(tpm_ctx* c) {
   TPM_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (err) {
     TPM_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    if (err & kErrRung) return fail(TPM_ERR_RUNG, "a new rung fell outside [0, 32) and was clamped");
-    return fail(TPM_ERR_INVALID, "|v * dt| >= 2^31 box lengths for some particle (left unmoved)");
+    return error_fail(err);
   }
   return TPM_OK;
 }

@@ -181,7 +181,7 @@ void dispatcher(tpm_server* s) {
       float ms = 0;
       if (rq.status == TPM_OK && cudaEventElapsedTime(&ms, sl.e0, sl.e1) == cudaSuccess) rq.device_ms = ms;
       if (rq.status == TPM_OK && *sl.err_host) {
-        rq.status = (*sl.err_host & kErrRung) ? TPM_ERR_RUNG : TPM_ERR_INVALID;
+        rq.status = error_status(*sl.err_host);
         *sl.err_host = 0;
       }
       ServeBox& bx = s->boxes[rq.box];

@@ -19,6 +19,13 @@ int fail(int status, const std::string& msg) {
   return status;
 }
 
+int error_fail(int err) {
+  const int status = error_status(err);
+  return fail(status, status == TPM_ERR_TIMEOUT ? "a bounded device wait (scan look-back) gave up"
+                      : status == TPM_ERR_RUNG  ? "a new rung fell outside [0, 32) and was clamped"
+                                                : "|v * dt| >= 2^31 box lengths for some particle (left unmoved)");
+}
+
 void stage_begin(tpm_ctx* c, Stage s) {
   if (!c->stage_timing) return;
   cudaEventRecord(c->ev.beg[s][c->ev.count[s] % kStageSlots], c->stream);
@@ -645,7 +652,7 @@ int tpm_kick_pme(tpm_ctx* c, const int* box, int min_rung, double scale, double 
   TPM_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (err) {
     TPM_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    if (err & kErrRung) return fail(TPM_ERR_RUNG, "a new rung fell outside [0, 32) and was clamped");
+    if (err & (kErrTimeout | kErrRung)) return error_fail(err);
   }
   return TPM_OK;
 }
@@ -660,7 +667,7 @@ int tpm_drift(tpm_ctx* c, double dt) {
   TPM_CUDA_TRY(cudaStreamSynchronize(c->stream));
   if (err) {
     TPM_CUDA_TRY(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream));
-    return fail(TPM_ERR_INVALID, "|v * dt| >= 2^31 box lengths for some particle (left unmoved)");
+    return error_fail(err);
   }
   return TPM_OK;
 }

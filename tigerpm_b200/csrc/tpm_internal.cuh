@@ -28,6 +28,9 @@ constexpr int kDepositFracBits = 40;
 constexpr int kErrRung = 1;
 constexpr int kErrBounds = 2;
 constexpr int kErrTimeout = 4;
+// The status of an error word that is not 0, worst first; error_fail adds its message.
+inline int error_status(int err) { return err & kErrTimeout ? TPM_ERR_TIMEOUT : err & kErrRung ? TPM_ERR_RUNG : TPM_ERR_INVALID; }
+int error_fail(int err);
 
 // Records a failure message for tpm_last_error_message and returns status.
 int fail(int status, const std::string& msg);
