@@ -1,7 +1,7 @@
 """The partition sort where its paths meet: particle counts on and beside a
 scan tile (4,096) and a shared-memory unit (8,192), boxes whose units are too
 large for one block (a share of the particles in one cell or one row), chain
-meshes of many shapes up to 260 cells a side, and a captured batch step
+meshes of many shapes up to 260 cells a side, far fewer particles than cells, and a captured batch step
 replayed.  Positions, velocities and rungs in the
 oracle's order, bit for bit."""
 import numpy as np
@@ -67,6 +67,22 @@ def test_chain_mesh_shapes(C):
 
 def test_large_chain_mesh():
     sort_and_check(with_random_motion(crowded(200003, 0.1, "row", 260, 5), 5), 260)
+
+
+@pytest.mark.parametrize("n,C", [(1000, 160), (3000, 160), (200003, 160), (200003, 200), (200003, 260), (2200000, 160)])
+def test_chain_mesh_finer_than_the_particles(n, C):
+    """Units of a few particles in a thousand cells each: sorted by the level kernels alone once there are many."""
+    ps = with_random_motion(W.uniform(n, C), C)
+    with TigerPM(make_options(max(2, round(n ** (1 / 3))), 16, chain=C), n) as t:
+        t.set_particles(ps)
+        before = t.launch_count()
+        t.chainmesh_create()
+        launches = t.launch_count() - before
+        check(ps, C, t)
+    levels = 3 * int(np.ceil(np.log2(C)))
+    many = n in (3000, 200003)
+    if many:  # keys, three of the cell counts' scan, cells of positions, two per level, gather
+        assert launches == 6 + 2 * levels
 
 
 def test_replayed_capture_sorts_new_input():

@@ -414,7 +414,8 @@ __global__ void __launch_bounds__(kScanThreads, 4)
         if (back >= 0 && nd.pm + back < nd.e) slot[nd.pm + back] = (int32_t)p;
       }
     }
-    __syncthreads();  // the tile's shared values are read before the next one's
+    if (tiles <= gridDim.x) return;  // a tile for every block: no other ticket
+    __syncthreads();                 // the tile's shared values are read before the next one's
   }
 }
 
@@ -790,19 +791,35 @@ int scan_exclusive(tpm_ctx* c, const int32_t* in, int64_t n, int32_t* out) {
 
 // Where k_finish takes over: the first node level whose nodes are expected to
 // fit its shared memory (0.8 of kUnit positions at the mean density, for the
-// widest node) with few enough cells.  udim < 0: no level does.
+// widest node) with few enough cells.  udim < 0: no level does, or the level
+// kernels are faster.
+//
+// A wave of units (two blocks on each of 148 SMs) takes 4.7 us per level
+// however few particles they hold, since each fills a table of its cells'
+// nodes; the level kernels take 18 us up to 5e5 particles and 22 us per 1e6
+// particles above (deep levels of fine meshes, where every position looks its
+// node up).  Hence units are taken up to four waves, or with at least 700
+// particles each; empty ones cost a block's start.  Sort with and without
+// them: 0.65 / 0.78 ms (8,000 particles, 128^3 cells, 1,024 units), 1.26 / 0.96
+// (200,003, 160^3, 2,560), 1.92 / 2.25 (4e6, 160^3), 2.86 / 2.65 (4e6, 200^3,
+// 6,400), 5.00 / 2.11 (200,003, 260^3, 16,640).
+constexpr int64_t kUnitsFew = 4 * 2 * 148, kUnitMean = 700;
+
 struct FinishStart {
   int udim = -1, ulevel = 0;
 };
 
 FinishStart finish_start(const tpm_ctx* c, int64_t n) {
-  const int C = c->C;
+  const int64_t C = c->C;
   for (int dim = 2; dim >= 0; dim--)
     for (int level = 0; level < c->max_depth1d; level++) {
-      const int64_t row = dim == 2 ? (int64_t)C * C : dim == 1 ? C : 1;
+      const int64_t row = dim == 2 ? C * C : dim == 1 ? C : 1;
       const int64_t cells = c->unit_levels[level].widest * row;
       const double mean = (double)n * (double)cells / ((double)C * C * C);
-      if (cells <= kUnitCells && (n <= kUnit || mean <= 0.8 * kUnit)) return {dim, level};
+      if (cells > kUnitCells || (n > kUnit && mean > 0.8 * kUnit)) continue;
+      const int64_t units = C * C / row * c->unit_levels[level].count;
+      if (std::min(units, n) + units / 128 > std::max(kUnitsFew, n / kUnitMean)) return {};
+      return {dim, level};
     }
   return {};
 }
