@@ -123,7 +123,7 @@ int tpm_check_errors(tpm_ctx* c) {
 
 int tpm_set_wait_limit(tpm_ctx* c, int64_t polls) {
   if (!c || polls < 0) return fail(TPM_ERR_INVALID, "null context or negative limit");
-  c->wait_polls = polls;
+  c->wait_polls = (int)std::min<int64_t>(polls, 0x7fffffff);
   return TPM_OK;
 }
 

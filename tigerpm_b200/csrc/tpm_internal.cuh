@@ -53,7 +53,7 @@ int fail(int status, const std::string& msg);
 constexpr int kSortCounters = 64, kSortGaveUp = 61, kSortBig = 62, kSortJumps = 63;
 
 // Polls of one look-back wait of the sort before it gives up (about a second).
-constexpr long long kWaitPolls = 1ll << 22;
+constexpr int kWaitPolls = 1 << 22;
 
 // Intervals of the 1-D bisection at one depth: their place among the context's
 // unit_cuts, their number and the widest one.
@@ -186,7 +186,7 @@ struct tpm_ctx {
   bool int_active = false;
 
   int* d_err = nullptr;
-  long long wait_polls = tpm::kWaitPolls;  // limit of the device waits (tpm_set_wait_limit)
+  int wait_polls = tpm::kWaitPolls;  // limit of the device waits (tpm_set_wait_limit)
   int64_t launches = 0;
   int64_t device_bytes = 0;
   tpm::StageEvents ev{};
