@@ -1,0 +1,54 @@
+"""The rounding of the mesh potential against 64 bits on boxes of a third of
+the mesh's points per side: an even random set, and a displaced lattice, whose
+own harmonics are the largest modes of the density.
+
+Bound: six line transforms of about nine butterflies each, each rounding to
+2^-24, add up at random to sqrt(54) 6e-8 / 2 = 2.2e-7 of the result's rms.
+Twice that is allowed, and 6e-7 for the lattices.  A part of the mean density
+left in low modes, where the potential is largest, breaks it."""
+import math
+
+import numpy as np
+import pytest
+
+import oracle as O
+from helpers import rel_rms
+from tigerpm_b200 import workloads as W
+from tigerpm_b200.api import GRAVITY_LONG_PME, Range, TigerPM, make_options
+
+pytestmark = pytest.mark.gpu
+
+
+def potential64(grid, rs_cells, x, y, z):
+    """The long-range potential in 64 bits: the oracle's cloud4 deposit, torch's transforms."""
+    import torch
+    k = torch.arange(grid, dtype=torch.float64, device="cuda")
+    k = torch.where(k < grid / 2, k, k - grid) * (2 * math.pi / grid)
+    half = torch.where(k == 0, torch.ones_like(k), 0.5 * k)
+    sinc = torch.where(k == 0, torch.ones_like(k), torch.sin(half) / half)
+    g = sinc ** -4 * torch.exp(-k * k * rs_cells ** 2)
+    h = grid // 2 + 1
+    spec = torch.fft.rfftn(torch.from_numpy(O.deposit(grid, 0, x, y, z)).cuda())
+    for i in range(grid):
+        k2 = (k * k)[i] + (k * k)[:, None] + (k * k)[None, :h]
+        if i == 0:
+            k2[0, 0] = 1.0
+        spec[i] *= -(g[i] * g[:, None] * g[None, :h]) / k2
+    spec[0, 0, 0] = 0
+    return torch.fft.irfftn(spec, s=(grid,) * 3).cpu().numpy()
+
+
+@pytest.mark.parametrize("grid,kind", [(g, "uniform") for g in (80, 96, 250, 400, 432, 480, 720)] +
+                         [(g, "zeldovich") for g in (80, 96, 250, 400, 480)])
+def test_potential_rounding(grid, kind):
+    side = grid // 3
+    ps = W.uniform(side ** 3, 7) if kind == "uniform" else W.zeldovich(side, 7, grid=side)
+    opts = make_options(side, grid, chain=max(3, grid // 10), rs_cells=2.0, deterministic_deposit=1)
+    with TigerPM(opts, ps.n) as t:
+        t.set_particles(ps)
+        t.chainmesh_create()
+        t.gravity_long_compute(GRAVITY_LONG_PME)
+        phi = t.gravity_long_get_phi(Range((0, 0, 0), (grid,) * 3))
+        x, y, z, *_ = t.get_particles()
+    err = rel_rms(phi, potential64(grid, 2.0, x, y, z))
+    assert err < (4.4e-7 if kind == "uniform" else 6e-7)

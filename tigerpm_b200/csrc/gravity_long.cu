@@ -92,6 +92,7 @@ struct DepositArgs {
   int N;
   int ntile;     // tiles per side
   double scale;  // 4 pi N (times the accumulator's fixed-point unit)
+  double mean;   // of rho: every particle's weights add up to 1
   float* __restrict__ rho;
 };
 
@@ -346,6 +347,11 @@ __global__ void __launch_bounds__(dep_threads<M>, 3) k_deposit(DepositArgs a) {
   __syncthreads();
   return false;
   };
+  // The stored density is without its mean.  The Green's function drops that
+  // mode, but in the transform its rounding (radix-5 butterflies and products
+  // with twiddles do not cancel a constant line exactly) falls on low modes,
+  // where the potential is largest: error against 64 bits of a random set at
+  // 400^3 2.1e-6 -> 2.3e-7, at 384^3 3.5e-6 -> 1.9e-7, at 768^3 1.1e-6 -> 2.2e-7.
   auto store_tile = [&](auto mode) {
     constexpr int MODE = decltype(mode)::value;
     using A = DepAcc<MODE>;
@@ -353,7 +359,7 @@ __global__ void __launch_bounds__(dep_threads<M>, 3) k_deposit(DepositArgs a) {
     for (int i = threadIdx.x; i < T * T * T; i += blockDim.x) {
       const int lz = i % T, ly = (i / T) % T, lx = i / (T * T);
       if (lx < ext[0] && ly < ext[1] && lz < ext[2])
-        a.rho[((int64_t)(o[0] + lx) * N + (o[1] + ly)) * N + (o[2] + lz)] = (float)A::value(acc[i], a.scale);
+        a.rho[((int64_t)(o[0] + lx) * N + (o[1] + ly)) * N + (o[2] + lz)] = (float)(A::value(acc[i], a.scale) - a.mean);
     }
   };
   if (deposit_tile(std::integral_constant<int, M>{})) {
@@ -440,6 +446,7 @@ int launch_deposit_T(tpm_ctx* c, DepositArgs a) {
   const int blocks = a.ntile * a.ntile * a.ntile;
   const size_t smem = sizeof(typename DepAcc<M>::T) * T * T * T + sizeof(int32_t) * dep_list<M>;
   a.scale = 4.0 * M_PI * c->N;
+  a.mean = a.scale * (double)c->n / ((double)c->N * c->N * c->N);
   switch (c->opt.assign) {
     case TPM_ASSIGN_CIC:
       TPM_CUDA_TRY(cudaFuncSetAttribute(k_deposit<T, TPM_ASSIGN_CIC, M>,
@@ -508,7 +515,7 @@ int gravity_long(tpm_ctx* c, int type) {
   a.C = c->C;
   a.N = N;
   a.ntile = 0;
-  a.scale = 0;
+  a.scale = a.mean = 0;
   a.rho = c->rho;
   int rc;
   // tile edge: 24 points on large meshes (fewer redundant particle visits),
