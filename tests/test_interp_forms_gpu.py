@@ -1,8 +1,9 @@
 """The long-range interpolation over the forms its kernels take: meshes whose
 rows are not whole quads, runs at every place of a quad and across the
 boundary, scalar tiles, sparse cells, cells split over many blocks, some sinks
-only, a kick box inside the mesh, and a batch of boxes of all kinds.  Forces
-against the oracle's FP64 kick on the same potential."""
+only, a kick box inside the mesh, the per-cell launch without the work queue, and
+a batch of boxes of all kinds.  Forces against the oracle's FP64 kick on the same
+potential; with and without the queue on the same bits of it."""
 import numpy as np
 import pytest
 
@@ -37,7 +38,7 @@ def test_forces(kind, n_side, grid, C, min_rung):
         t.kick_pme_begin(min_rung, 1.0, 0.01, False)
         t.kick_pme_end()
         G = np.stack(t.get_forces(), 1)
-        # the same through the per-cell launch (no queue) and through a box of cells
+        # the same through a box of cells
         t.set_particles(ps)
         t.chainmesh_create()
         t.gravity_long_compute(GRAVITY_LONG_PME)
@@ -52,6 +53,35 @@ def test_forces(kind, n_side, grid, C, min_rung):
     x, y, z = key % C, key // C % C, key // (C * C)
     inside = due & (x >= 1) & (y < C - 1) & (z == 1)
     assert rel_rms(B[inside], OG[inside]) < 2e-5 and not np.any(B[~inside])
+
+
+@pytest.mark.parametrize("kind,n_side,grid,C", [
+    ("uniform", 24, 30, 5), ("uniform", 24, 45, 7), ("uniform", 20, 64, 6), ("uniform", 24, 16, 3), ("uniform", 30, 100, 11),
+    ("halos", 32, 48, 6), ("halos", 32, 64, 12)])
+def test_without_the_queue(kind, n_side, grid, C):
+    """kick_grid = 1: no queue, whole cells in the staged tile, the direct form and the scalar one.  The split cells'
+    sinks take another form in the queue's run, so forces agree to the rounding of the interpolation's sums."""
+    ps = with_random_motion(particle_set(kind, n_side, 3), 3)
+    opts = make_options(n_side, grid, chain=C, rs_cells=grid / C / 4.5, rcut_over_rs=4.5, deterministic_deposit=1)
+    G = []
+    for kick_grid in (0, 1):
+        opts.kick_grid = kick_grid
+        with TigerPM(opts, ps.n) as t:
+            t.set_particles(ps)
+            t.chainmesh_create()
+            before = t.get_particles()
+            offs = t.chainmesh_offsets()
+            t.gravity_long_compute(GRAVITY_LONG_PME)
+            phi = t.gravity_long_get_phi(Range((0, 0, 0), (grid,) * 3))
+            t.kick_pme_begin(0, 1.0, 0.01, False)
+            t.kick_pme_end()
+            G.append(np.stack(t.get_forces(), 1))
+    OG = oracle_forces(opts, before, phi, offs, 0)
+    assert rel_rms(G[1][:, :3], OG[:, :3]) < 1e-5 and rel_rms(G[1][:, 3], OG[:, 3]) < 1e-5
+    if kind == "uniform":  # no cell is split: the same kernels
+        assert np.array_equal(G[0].view(np.uint32), G[1].view(np.uint32))
+    else:
+        assert rel_rms(G[0], G[1]) < 1e-6
 
 
 def test_batch_of_all_kinds():

@@ -1,7 +1,8 @@
 """The partition sort where its paths meet: particle counts on and beside a
 scan tile (4,096) and a shared-memory unit (8,192), boxes whose units are too
 large for one block (a share of the particles in one cell or one row), chain
-meshes of many shapes up to 260 cells a side, far fewer particles than cells, and a captured batch step
+meshes of many shapes up to 260 cells a side, far fewer particles than cells,
+sets large enough for the gather's records, and a captured batch step
 replayed.  Positions, velocities and rungs in the
 oracle's order, bit for bit."""
 import numpy as np
@@ -67,6 +68,22 @@ def test_chain_mesh_shapes(C):
 
 def test_large_chain_mesh():
     sort_and_check(with_random_motion(crowded(200003, 0.1, "row", 260, 5), 5), 260)
+
+
+def test_no_unit_fits_a_block():
+    """Thousands of particles in every chain cell (the reference's default options): the level kernels alone."""
+    sort_and_check(with_random_motion(W.uniform(200003, 8), 8), 3)
+
+
+def test_gather_of_many_particles_in_no_order():
+    """Above 4,194,304 particles the gather reads records where most sources lie apart, as in a random set; the set
+    sorted once more is in order, and is gathered from the arrays."""
+    ps = with_random_motion(W.uniform(4300003, 9), 9)
+    with TigerPM(make_options(163, 16, chain=37), ps.n) as t:
+        t.set_particles(ps)
+        for _ in range(2):
+            t.chainmesh_create()
+            check(ps, 37, t)
 
 
 @pytest.mark.parametrize("n,C", [(1000, 160), (3000, 160), (200003, 160), (200003, 200), (200003, 260), (2200000, 160)])
