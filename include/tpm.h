@@ -118,9 +118,9 @@ typedef struct tpm_options {
   int fft_group;       /* x-planes per launch of the library FFT's z / y passes
                         * (0: all; smaller groups keep the spectrum in L2 between
                         * the two passes) */
-  int kick_grid;       /* 0: the PP + kick as one persistent launch over a cost-sorted
-                        * queue of (cell, sink pass) items (default; balances clustered
-                        * boxes); 1: one block per sink cell */
+  int kick_grid;       /* 0: cells of many sinks as (cell, sink pass) items of a
+                        * cost-sorted queue, all others one block per cell (default;
+                        * balances clustered boxes); 1: one block per sink cell */
 } tpm_options;
 
 typedef struct tpm_ctx tpm_ctx;
@@ -135,7 +135,8 @@ typedef struct tpm_stage_times {
   float kick_ms;
   float drift_ms;
   float ewald_ms;
-  float interp_ms; /* long-range interpolation at the sinks (part of the kick) */
+  float interp_ms; /* the kick's work queue and the long-range interpolation at the
+                    * sinks (a part of the kick that kick_ms does not contain) */
 } tpm_stage_times;
 
 /* Device addresses of the context's particle arrays (current order). */
@@ -423,10 +424,10 @@ int tpm_growth_factor(double omega_m, double a, double* out);
  * over the launch (src/kick_pme.cu:139-141) and box splitting when device
  * memory is short (src/kick_pme.cu:418-430).  A batch step runs every box's
  * chain-mesh sort and long-range solve concurrently (one stream per box),
- * then the interpolation of all boxes in one launch and the PP sum + rung
- * kick of all boxes in ONE persistent launch over a work queue of
- * (box, chain cell) items ordered heaviest first.  Each box is a tpm_ctx
- * reachable through tpm_batch_box (results, forces, particles). */
+ * then the interpolation and the PP sum + rung kick of all boxes in two
+ * launches each: one over the chain cells of every box, one over a work queue
+ * of the passes of cells of many sinks, ordered heaviest first.  Each box is a
+ * tpm_ctx reachable through tpm_batch_box (results, forces, particles). */
 typedef struct tpm_batch tpm_batch;
 
 /* Launch shape of the kick kernel: warps per block, sources staged in
@@ -445,7 +446,7 @@ typedef struct tpm_batch_times {
   float long_range_ms; /* fork: every box's sort + deposit + FFT solve */
   float queue_ms;      /* work-queue build */
   float interp_ms;     /* long-range interpolation, all boxes */
-  float kick_ms;       /* persistent PP + rung kick, all boxes */
+  float kick_ms;       /* PP + rung kick, all boxes */
 } tpm_batch_times;
 
 #define TPM_BATCH_RESTORE 1 /* restore every box's particles from its input first */

@@ -137,10 +137,9 @@ def test_force_at():
 
 # The library's own transforms (fft3d.cu) run for grids that are multiples of
 # 16 made of the radices 16, 8, 4, 3, 5 and 2: the generic block engine for
-# every such grid (fft="block"), the warp-per-line engine by default where the
-# grid has a compiled line plan (96, 128, 160 here; 48 and 80 have none and
-# take the block engine).  Each is compared against both the oracle and cuFFT
-# on the same deposit.
+# every such grid (fft="block"), the line engine by default where the grid has a
+# compiled line plan (all of these).  Each is compared against both the oracle
+# and cuFFT on the same deposit.
 @pytest.mark.parametrize("fft", ["auto", "block"])
 @pytest.mark.parametrize("grid", [48, 80, 96, 128, 160])
 def test_library_fft_matches_oracle_and_cufft(grid, fft):

@@ -1,5 +1,5 @@
 """The line plans whose lines do not fill a warp evenly (400, 432, 720 points:
-20, 18 and 24 lanes) and the other plans beside the power-of-two ones, against
+20, 36 and 24 lanes) and the other plans beside the power-of-two ones, against
 the block engine and cuFFT on one exact deposit."""
 import pytest
 

@@ -11,13 +11,14 @@
 //           chain-mesh sort, deposit and the FFT Poisson solve; the boxes'
 //           kernels overlap on the device
 //   join    the main stream waits for all boxes
-//   queue   every non-empty (box, chain cell) becomes a work item, bucketed
-//           by the binary order of magnitude of its cost (sinks x
-//           neighbourhood sources), heaviest bucket first
+//   queue   the sink passes of every (box, chain cell) of many sinks become
+//           work items, bucketed by the binary order of magnitude of their
+//           cost (sinks x neighbourhood sources), heaviest bucket first
 //   interp  long-range interpolation: one launch over the cells, one over the
 //           pass items of split cells
-//   kick    ONE persistent launch: resident blocks take items from a global
-//           counter until the queue is empty (PP sum + rung kick)
+//   kick    (PP sum + rung kick) a persistent launch, whose resident blocks take
+//           the split cells' items from a global counter until the queue is
+//           empty, and one over the other cells
 //
 // With TPM_BATCH_GRAPH the whole step is captured once as a CUDA graph (the
 // fork becomes parallel branches) and replayed; a new capture is made when

@@ -22,12 +22,13 @@
 // columns are zero and never reach phi).  Two engines run the passes:
 //
 //  * line engine (the meshes with a compiled plan, TPM_LINE_SIZES): one line
-//    per TL lanes of a warp, E = N / TL values per lane in registers, a
-//    compile-time Stockham plan of radices 16/12/10/8/6/5/4/3/2 that divide E
-//    (three stages for most sizes: 12.8.8 at 768, 12.8.4 at 384), the line's
-//    row of shared memory between stages with warp-level synchronisation only,
-//    and per-stage twiddle tables; the x pass runs its inverse with the
-//    reversed plan straight from the forward transform's registers;
+//    per TL threads, E = N / TL values per thread in registers, a compile-time
+//    Stockham plan of radices 16/12/10/8/6/5/4/3/2 that divide E (three stages
+//    for most sizes: 12.8.8 at 768, 12.8.4 at 384), the line's row of shared
+//    memory only between stages, and per-stage twiddle tables; the y and x
+//    passes read and write their columns straight from and to global memory,
+//    and the x pass runs its inverse with the reversed plan straight from the
+//    forward transform's registers;
 //  * block engine (every other supported N): each block holds 4 lines in
 //    shared memory and transforms them with a radix-16/8/4/3/5/2 Stockham FFT
 //    over two shared buffers.
@@ -467,15 +468,18 @@ __global__ void __launch_bounds__(kFftThreads) k_fft_z_c2r(const float2* __restr
 // ------------------------------------------------------------ line engine
 //
 // The same five passes for the mesh sizes that have a compile-time plan:
-// one line of length N is held by TL lanes of a warp (TL = 4 .. 32), E = N / TL
-// values per lane in registers.  A Stockham stage of radix R (R divides E)
-// gives every lane E / R butterflies j = lane + TL b; between stages the
-// line goes through its own row of shared memory with only warp-level
-// synchronisation, and the first stage reads its inputs (global rows, or the
-// block's transposed columns) and the last stage writes its outputs in
-// natural order straight from registers.  Radices, strides and divisions are
-// compile-time constants.  Column passes stage kLineCols = 8 neighbouring
-// columns per block (64-byte row segments) through shared memory.
+// one line of length N is held by TL threads (TL = 4 .. 36), E = N / TL values
+// each in registers.  A Stockham stage of radix R (R divides E) gives every
+// thread E / R butterflies j = lane + TL b; between stages the line goes through
+// its own row of shared memory, the first stage reads its inputs and the last
+// stage writes its outputs in natural order straight from and to global
+// memory.  Radices, strides and divisions are compile-time constants.  A block
+// has kLineCols = 8 lines.  In the z passes a line's threads are neighbours:
+// they share a warp where TL is a power of two, and the exchange is then a
+// warp's own; else (TL = 20, 24, 36) it takes a block barrier.  In the column
+// passes neighbouring threads have neighbouring columns (64-byte row segments),
+// a line's threads are spread over the block, and every exchange is a block
+// barrier.
 constexpr int kLineCols = 8;
 
 struct LinePlan {
@@ -915,8 +919,10 @@ int line_poisson(tpm_ctx* c, float2* Y, int Sz, const float* gt, float norm) {
   return TPM_OK;
 }
 
-// Mesh sizes with a compiled line plan (the benchmark meshes, the batched
-// and served box meshes, and the powers of two up to 1024).
+// Mesh sizes with a compiled line plan: every size the block engine takes from
+// 48 to 768 points, and 1024.  The rest run the block engine: 16 and 32 points,
+// where the passes are all launch (z and y together 16 us), and 800, 864 and 960,
+// for which no line plan has been measured.
 #define TPM_LINE_SIZES(X) \
   X(48) X(64) X(80) X(96) X(128) X(144) X(160) X(192) X(240) X(256) X(288) X(320) X(384) X(400) X(432) X(480) X(512) X(576) X(640) X(720) X(768) X(1024)
 

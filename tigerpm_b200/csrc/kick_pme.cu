@@ -243,11 +243,13 @@ __device__ __forceinline__ void interp_long(const KickArgs& a, int4 q, float& lx
 
 // The same with the z weights in pairs (packed FMAs) and the loop over planes
 // unrolled, its weights in registers instead of local memory: at 128 registers
-// and 8 resident 64-thread blocks it replaces the form above at 85 registers
+// and 8 resident 64-thread blocks it replaces the form above at 80 registers
 // and 12 where the arguments are kernel parameters (2.98 against 3.07 ms at
 // 256^3 on a 768^3 mesh, 0.28 against 0.33 ms with a quarter of 128^3 sinks due,
 // 24 against 28 us at 32^3); with 12 blocks it spills (3.92 ms).  Runs that
-// wrap in z, and meshes whose rows are not whole quads, take the form above.
+// wrap in z, and meshes whose rows are not whole quads, take the form above, at
+// 8 blocks too: a kernel of its own with 12 took 75 against 65 us (60^3 sinks on
+// a 90^3 mesh), 91 against 80 (64^3 on 130^3), 552 against 559 (128^3 on 190^3).
 __device__ __forceinline__ void interp_packed(const KickArgs& a, int4 q, float& lx, float& ly, float& lz,
                                             float& lp) {
   const int N = a.N;
@@ -929,7 +931,7 @@ __device__ __forceinline__ void kick_cell(const KickArgs& a, int cx, int cy, int
     // 2. long-range interpolation and the kick, one thread per sorted sink
     for (int e = tid; e < nact; e += T) {
       const int32_t i = sbase + (int32_t)sidx[e];
-      const float lx = a.gx[i], ly = a.gy[i], lz = a.gz[i], lp = a.pot[i];  // from k_interp_long
+      const float lx = a.gx[i], ly = a.gy[i], lz = a.gz[i], lp = a.pot[i];  // from the interpolation kernels
       const float* A = acc + e * 8;
       // pair sums back from units of 2 r_s: force x (1/2r_s)^2, potential x 1/2r_s
       const float fs = a.inv2rs * a.inv2rs * kLog2e;
@@ -1199,7 +1201,7 @@ __global__ void __launch_bounds__(64, 8)
 // every box's cells in natural order, so that neighbouring cells' stencil
 // reads share the L1 and L2 as in the single-box k_interp_direct (in the
 // queue's cost order, items of different boxes interleave).
-// 12 resident 64-thread blocks per SM (85 registers): with the arguments of its
+// 12 resident 64-thread blocks per SM (80 registers): with the arguments of its
 // box in registers the packed form is slower here (0.85 against 0.77 ms for 12
 // boxes of 32^3 to 96^3).
 __global__ void __launch_bounds__(64, 12)
@@ -1337,13 +1339,17 @@ int kick_pme(tpm_ctx* c, const int box[6], int min_rung, double scale, double t0
   auto kern = wrap ? k_kick_pme<true, false> : c->rcut_box > 0 ? k_kick_pme<false, true> : k_kick_pme<false, false>;
   TPM_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const bool queue = ncell > 0 && !c->opt.kick_grid;
+  stage_begin(c, kStInterp);  // the queue too: the interpolation is the first to use it
   if (queue) {
     const int rc = kick_queue_build(c, a, k, b, e);
     if (rc) return rc;
   }
   const int* cls = queue ? c->kq.d_class : nullptr;
-  // Where the mean cell is one that the queue splits, the cells are alike and
-  // need no balancing: the interpolation takes them whole.
+  // Where the mean cell is one that the queue splits, nearly every cell would
+  // be left to the items, which do not use the staged tile: the interpolation
+  // takes all of them whole, the heavy ones of a clustered set too (0.64 ms at
+  // 300,000 clustered particles in 5^3 cells, 1.5 ms at 100,000 in 3^3, against
+  // 31 and 15 ms for their pairs).
   const bool apart = queue && mean_cell <= (double)kSplitPasses * k.npass;
   // Long-range interpolation.  A shared-memory tile of phi pays when a chain
   // cell's reach (its mesh span + 5 points per dim) is small against its
@@ -1353,7 +1359,6 @@ int kick_pme(tpm_ctx* c, const int box[6], int min_rung, double scale, double t0
   const int maxw = (c->N + C - 1) / C + 8;
   const size_t tile_bytes = sizeof(float) * (size_t)maxw * maxw * maxw;
   const double span = (double)c->N / C + 6.0;
-  stage_begin(c, kStInterp);
   if (ncell > 0) {
     if (tile_bytes <= 48 * 1024 && span * span * span <= 16.0 * mean_cell) {
       k_interp_tile<<<(unsigned)ncell, 128, tile_bytes, c->stream>>>(a, maxw, apart ? cls : nullptr);
